@@ -261,9 +261,9 @@ def work(case):
 
 def tolerance(case):
     """fp32: the order of the sums (a weight gradient summed one by one over 16384 tokens is 2.3e-6 off its value in
-    64 bits, over 65536 tokens 4.6e-6; single elements by 5e-5 of the root mean square, in a whole step 7e-5).  bf16: the rounding of activations and their gradients (measured against the same step in fp32: up to 7e-3
-    on moments and 1e-2 on logits; single elements of the moments that are sums of much larger ones differ by
-    about their root mean square)."""
+    64 bits, over 65536 tokens 4.6e-6; four times that).  bf16: the rounding of activations and their gradients
+    (measured against the same step in fp32: up to 7e-3 on moments and 1e-2 on logits).  Single elements of the
+    moments that are sums of much larger ones differ by up to 200 times the relative error of the whole."""
     if case["dtype"] == "f32":
-        return {"rel": 1.8e-5, "max": 5e-4}
+        return {"rel": 1.8e-5, "max": 3e-3}
     return {"rel": 0.03, "max": 0.99}
