@@ -13,6 +13,7 @@ import math
 
 import numpy as np
 import torch
+import torch.utils.checkpoint
 
 from alpha2_b200.autograd import Param, Tape
 from alpha2_b200.backend import CudaBackend, TensorData
@@ -267,3 +268,100 @@ def tolerance(case):
     if case["dtype"] == "f32":
         return {"rel": 1.8e-5, "max": 3e-3}
     return {"rel": 0.03, "max": 0.99}
+
+
+def _norm64(x, w, prefix, rms):
+    if not rms:
+        x = x - x.mean(-1, keepdim=True)
+    x = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w[prefix + ".weight"]
+    return x if rms else x + w[prefix + ".bias"]
+
+
+def _rotate64(x):
+    """Rotary embedding, halves rotated, of x [B, H, T, D]."""
+    T, D = x.shape[2:]
+    angle = torch.arange(T, dtype=torch.float64, device="cuda")[:, None] * \
+        10000.0 ** (-torch.arange(0, D, 2, dtype=torch.float64, device="cuda") / D)
+    c, s = torch.cos(angle), torch.sin(angle)
+    a, b = x[..., :D // 2], x[..., D // 2:]
+    return torch.cat([a * c - b * s, b * c + a * s], -1)
+
+
+def _layer64(x, w, p, heads, swiglu):
+    B, T, E = x.shape
+    qkv = (_norm64(x, w, p + ".ln1", swiglu) @ w[p + ".attn.wqkv"].T).view(B, T, 3, heads, E // heads)
+    q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))
+    if swiglu:
+        q, k = _rotate64(q), _rotate64(k)
+    s = 30.0 * torch.tanh(q @ k.transpose(-1, -2) / math.sqrt(E // heads) / 30.0)
+    s = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), -math.inf)
+    x = x + (s.softmax(-1) @ v).transpose(1, 2).reshape(B, T, E) @ w[p + ".attn.wo"].T
+    h = _norm64(x, w, p + ".ln2", swiglu)
+    if swiglu:
+        h = torch.nn.functional.silu(h @ w[p + ".mlp.fc_gate"].T) * (h @ w[p + ".mlp.fc_up"].T)
+        return x + h @ w[p + ".mlp.fc_proj"].T
+    h = torch.nn.functional.gelu(h @ w[p + ".mlp.fc1"].T, approximate="tanh")
+    return x + h @ w[p + ".mlp.fc2"].T
+
+
+def _hidden64(case, w, tokens):
+    swiglu = case["arch"] == "swiglu"
+    x = w["wte"][tokens]
+    if not swiglu:
+        x = x + w["wpe"][:tokens.shape[1]]
+    for i in range(case["layers"]):
+        x = torch.utils.checkpoint.checkpoint(_layer64, x, w, f"layer.{i}", case["heads"], swiglu, use_reentrant=False)
+    return _norm64(x, w, "lnF", swiglu)
+
+
+def exact(case, seed):
+    """The same step or logits in 64 bits (from the fp32 weights, also where the layers compute in bf16).  A
+    generation has no such value: one near-tie sampled otherwise changes all that follows."""
+    if case["kind"] == "sample" or work(case)["flops"] > 4e13:
+        return None
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    shapes = _shapes(_config(case))
+    flat = _Flat(shapes)
+    for name, shape in shapes:
+        if len(shape) == 2:
+            flat.torch(name).normal_(0.0, 0.02, generator=g)
+        elif name.endswith(".weight"):
+            flat.torch(name).fill_(1.0)
+    train = case["kind"] == "train"
+    w = {n: flat.torch(n).double().view(s).requires_grad_(train) for n, s in shapes}
+    head = w["wte"] if case["tied"] else w["lmHead"]
+    batches = [tuple(torch.as_tensor(a, device="cuda").long() for a in pair)
+               for pair in zipf_batches(seed, case.get("accum", 1), case["batch"], case["seq"], case["vocab"])]
+    B, T, E = case["batch"], case["seq"], case["width"]
+    # sequences at a time: layer inputs, one layer's intermediates and the logits within about 30 GB
+    at_once = max(1, int(4e9 / (T * (E * (case["layers"] + 40) + 8 * case["heads"] * T + 4 * case["vocab"]))))
+    if not train:
+        with torch.no_grad():
+            rows = [_hidden64(case, w, t)[:, -1:] if case["kind"] == "next" else _hidden64(case, w, t)
+                    for t in batches[0][0].split(at_once)]
+            return {"logits": torch.cat([r @ head.T for r in rows])}
+    loss = 0.0
+    for tokens, targets in batches:
+        for t, y in zip(tokens.split(at_once), targets.split(at_once)):
+            logits = _hidden64(case, w, t) @ head.T
+            part = torch.nn.functional.cross_entropy(logits.flatten(0, 1), y.flatten(), reduction="sum")
+            part = part / (B * T * case["accum"])
+            part.backward()
+            loss += part.item()
+            del logits, part
+    with torch.no_grad():
+        c = TrainConfig(batchSize=B, gradAccumSteps=case["accum"])
+        low, warm = c.lr / 10, min(2000, c.iters // 5)
+        lr = low + (c.lr - low) / warm
+        norm = math.sqrt(sum(float((p.grad ** 2).sum()) for p in w.values()))
+        clip = min(1.0, c.gradClip / norm)
+        out = {k: torch.zeros(flat.all.numel(), dtype=torch.float64, device="cuda") for k in ("weights", "m", "v")}
+        for name, shape in shapes:
+            p, d = w[name], w[name].grad * clip
+            if len(shape) == 2 and name not in ("wte", "wpe"):
+                p = p * (1 - lr * c.weightDecay)
+            at = flat.at[name][0]
+            for k, x in (("weights", p - lr * d / (d.abs() + c.eps)), ("m", (1 - c.beta1) * d),
+                         ("v", (1 - c.beta2) * d * d)):
+                out[k][at:at + x.numel()] = x.flatten()
+    return {"loss": loss if case["read_back"] else torch.tensor([loss], dtype=torch.float64, device="cuda"), **out}
