@@ -1,7 +1,8 @@
-// fp32 GEMM on the FMA pipes: the full-precision mode used by the fp32 parity
-// configurations (the reference accumulates each dot product in a double and rounds once,
-// packages/tensor/src/cpu_ref.ts:246-254; bf16 tensor-core products cannot meet a 1e-4
-// parameter tolerance, fp32 FMA accumulation does).  Arbitrary element strides cover the
+// Entry of the fp32 GEMM, the full-precision mode used by the fp32 parity configurations (the
+// reference accumulates each dot product in a double and rounds once,
+// packages/tensor/src/cpu_ref.ts:246-254).  The products run on the tensor cores as sums of
+// exact bf16 term products (gemm_f32_tc.cu); the kernel here, on the FMA pipes, takes what that
+// one does not: an empty sum (K = 0, epilogues included) and outputs of more than 2^25 tiles.  Arbitrary element strides cover the
 // three layouts of the Backend interface — A*B, A*B^T (matmulTransposed) and A^T*B
 // (matmulTransposedA), packages/core/src/interfaces.ts:53,111-112 — and batched matmul
 // with broadcastable batch strides for the unfused attention branch
@@ -104,11 +105,22 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(GemmF32Args g) {
   }
 }
 
+int gemm_f32_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M, int64_t N, int64_t K, int64_t lda,
+                       int64_t ldb, int64_t ldc, int epilogue, alpha_buf aux, int64_t ld_aux, int accumulate,
+                       int64_t batch, int64_t stride_a, int64_t stride_b, int64_t stride_c);
+
 int gemm_f32_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M, int64_t N, int64_t K, int64_t lda,
                     int64_t ldb, int64_t ldc, int epilogue, alpha_buf aux, int64_t ld_aux, int accumulate,
                     int64_t batch, int64_t stride_a, int64_t stride_b, int64_t stride_c) {
   if (M == 0 || N == 0 || batch == 0) return 0;
   ProfScope prof(PROF_GEMM_F32, 2.0 * (double)M * (double)N * (double)K * (double)batch);
+  ALPHA_CHECK(layout >= ALPHA_GEMM_NT && layout <= ALPHA_GEMM_TN, "alpha_gemm: bad layout %d", layout);
+  ALPHA_CHECK(batch <= 65535, "alpha_gemm: batch %lld > 65535", (long long)batch);
+  ALPHA_CHECK((M + TM - 1) / TM <= 65535, "alpha_gemm: M too large for the fp32 kernel");
+  // 32-bit tile counts and coordinates in the tensor-core kernel; an empty sum has no K step
+  if (K > 0 && N < (1 << 30) && K < (1 << 30) && ((M + 127) / 128) * ((N + 63) / 64) * batch < (1 << 25))
+    return gemm_f32_tc_launch(layout, A, B, C, M, N, K, lda, ldb, ldc, epilogue, aux, ld_aux, accumulate, batch, stride_a,
+                              stride_b, stride_c);
   GemmF32Args g;
   g.A = ptr<float>(A);
   g.B = ptr<float>(B);
@@ -122,11 +134,8 @@ int gemm_f32_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M
   switch (layout) {
     case ALPHA_GEMM_NT: g.sam = lda; g.sak = 1; g.sbk = 1; g.sbn = ldb; break;   // B stored [N,K]
     case ALPHA_GEMM_NN: g.sam = lda; g.sak = 1; g.sbk = ldb; g.sbn = 1; break;   // B stored [K,N]
-    case ALPHA_GEMM_TN: g.sam = 1; g.sak = lda; g.sbk = ldb; g.sbn = 1; break;   // A stored [K,M]
-    default: return set_error("alpha_gemm: bad layout %d", layout);
+    default:            g.sam = 1; g.sak = lda; g.sbk = ldb; g.sbn = 1; break;   // A stored [K,M]
   }
-  ALPHA_CHECK(batch <= 65535, "alpha_gemm: batch %lld > 65535", (long long)batch);
-  ALPHA_CHECK((M + TM - 1) / TM <= 65535, "alpha_gemm: M too large for the fp32 kernel");
   dim3 grid((unsigned)((N + TN - 1) / TN), (unsigned)((M + TM - 1) / TM), (unsigned)batch);
   gemm_f32_kernel<<<grid, 256, 0, g_stream>>>(g);
   ALPHA_LAUNCHED();

@@ -1,0 +1,527 @@
+// fp32 GEMM on the 5th-generation tensor cores without loss of precision: every fp32 operand
+// element is taken apart into three bf16 terms, x = h + m + l (round to nearest each, 8 bits of
+// significand per term, so the three hold all 24 bits), and the product is the sum of the six
+// term products of weight 2^-16 and above: l*h, h*l, m*m, m*h, h*m, h*h.  What is left out
+// (m*l, l*m, l*l) is below 2^-26 of |a*b|, a quarter of the rounding of one fp32 addition.
+//
+// Sums: the tensor core adds the 24 products-by-16 of one K step of 64 into a tensor-memory
+// accumulator, smallest terms first, and the epilogue warps add that partial sum into fp32
+// registers (round to nearest).  A dot product over K is therefore a chain of K/64 rounded
+// additions where an FMA loop has one of K, and the tensor core's truncating adds never see a
+// sum longer than 64 terms.  Error against 64 bits: tests/test_gpu_gemm_f32.py.
+//
+// Shape of the kernel: persistent, one CTA per SM, tile 128 x BN x 64, 16 warps (128 registers each):
+//   warps 0-7   operands: 16-byte global loads (both contiguity directions, coalesced), split in
+//               registers, written as three 128B-swizzled bf16 planes per operand.  The loads of
+//               the next K step are issued as soon as a register has been split.
+//   warps 8-15  accumulation: tensor memory -> registers after every K step (two accumulators
+//               alternate), epilogue at the end of the tile through shared memory, so that rows
+//               leave in 128-byte segments.  Warp 8 also issues the MMAs (one elected lane), a K step
+//               ahead of the one whose sums it is about to read.
+// The split happens in the kernel: done in a pass of its own it would read 4 and write 6 bytes per
+// element and operand, which costs a third of the GEMM's own time at K = 384.
+//
+// Infinities: inf splits into inf and NaN terms, and |x| >= 2^127 may round up to inf.  The operand
+// warps flag such a tile, and its elements that came out non-finite are recomputed with an fmaf
+// chain in K order.  NaN operands need nothing: the result is NaN either way.
+//
+// Measured on a B200: 8192 x 4096 x 384 in 248 us (104 TFLOP/s), 16384 x 768 x 256 in 82 us (79); an
+// FMA-pipe kernel with 4 x 4 outputs per thread ran such products at 9 to 15 TFLOP/s.  Bound by the operand
+// warps (splitting and the loads it waits for), not by the tensor core.
+#include <string.h>
+
+#include "tc_common.cuh"
+
+namespace alpha {
+
+using namespace tc;
+
+struct GemmF32TcArgs {
+  const float *A, *B;
+  float *C;             // output, or the split-K workspace (dense [split][batch][M][N])
+  const float *aux_in;
+  float *aux_out;
+  int64_t lda, ldb, ldc, ld_aux;
+  int64_t batch_a, batch_b, batch_c;
+  int64_t split_c;      // elements between two splits' slabs
+  int M, N, K;
+  int tiles_m, tiles_n, splits, kb_per_split, kblocks, batch;
+  int epilogue, accumulate;
+  int vec_a, vec_b, vec_c;   // 16-byte accesses are legal for A / B / (C and aux)
+  uint32_t *err;
+};
+
+constexpr int F3_BM = 128, F3_BK = 64, F3_STAGES = 2;
+constexpr int F3_OP_WARPS = 8, F3_ACC_WARPS = 8;
+constexpr int F3_THREADS = 32 * (F3_OP_WARPS + F3_ACC_WARPS);
+constexpr int F3_FLAGS = 8;   // ring of per-tile "holds an infinity" tags
+
+template <int BN>
+struct F3Layout {
+  static constexpr int A_PLANE = F3_BM * F3_BK * 2, B_PLANE = BN * F3_BK * 2;
+  static constexpr int STAGE = 3 * (A_PLANE + B_PLANE);
+  static constexpr int EPI_OFF = F3_STAGES * STAGE;
+  static constexpr int BAR_OFF = EPI_OFF + F3_ACC_WARPS * 4096;
+  static constexpr int TOTAL = BAR_OFF + 8 * (2 * F3_STAGES + 4) + 8 + 4 * F3_FLAGS;
+  static constexpr int DYN = TOTAL + 1024;   // slack to align the base to 1024 B
+};
+
+// x = h + m + l for a pair; each result holds the pair's two bf16 terms
+__device__ __forceinline__ void split3(float x0, float x1, uint32_t &h, uint32_t &m, uint32_t &l) {
+  h = bf16x2_pack(x0, x1);
+  const float r0 = x0 - __uint_as_float(h << 16), r1 = x1 - __uint_as_float(h & 0xFFFF0000u);
+  m = bf16x2_pack(r0, r1);
+  l = bf16x2_pack(r0 - __uint_as_float(m << 16), r1 - __uint_as_float(m & 0xFFFF0000u));
+}
+
+// One operand tile of ROWS (M or N) x 64 (K) on its way from global to shared memory, shared by
+// the 256 threads of the operand warps, four consecutive elements of the contiguous direction
+// per thread and pass.
+template <bool MN, int ROWS>
+struct F3Operand {
+  static constexpr int PASSES = ROWS * F3_BK / 4 / (32 * F3_OP_WARPS);
+  static constexpr int PLANE = ROWS * F3_BK * 2;
+  float4 r[PASSES];
+
+  __device__ __forceinline__ static int row_of(int tid, int i) {
+    return MN ? (tid % (ROWS / 4)) * 4 : i * 16 + tid / 16;
+  }
+  __device__ __forceinline__ static int k_of(int tid, int i) {
+    return MN ? i * (1024 / ROWS) + tid / (ROWS / 4) : (tid % 16) * 4;
+  }
+  __device__ __forceinline__ void load(const float *p, int64_t ld, int r0, int rows, int k0, int K, int vec, int tid) {
+#pragma unroll
+    for (int i = 0; i < PASSES; i++) {
+      const int row = r0 + row_of(tid, i), k = k0 + k_of(tid, i);
+      const int c = MN ? row : k, c_end = MN ? rows : K;        // contiguous coordinate and its limit
+      const bool in = MN ? k < K : row < rows;
+      const float *src = p + (MN ? (int64_t)k * ld + row : (int64_t)row * ld + k);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (vec && in && c + 4 <= c_end) {
+        v = *reinterpret_cast<const float4 *>(src);
+      } else if (in) {
+        if (c < c_end) v.x = src[0];
+        if (c + 1 < c_end) v.y = src[1];
+        if (c + 2 < c_end) v.z = src[2];
+        if (c + 3 < c_end) v.w = src[3];
+      }
+      r[i] = v;
+    }
+  }
+  // Returns whether the thread's elements hold an infinity or a value from 2^127 on.
+  __device__ __forceinline__ bool store(uint8_t *planes, int tid) const {
+    bool big = false;
+#pragma unroll
+    for (int i = 0; i < PASSES; i++) {
+      const int row = row_of(tid, i), k = k_of(tid, i);
+      // K-major: rows of 64 k (128 bytes); MN-major: atoms of 64 rows, per atom one 128-byte line per k
+      const uint32_t line = MN ? (uint32_t)((row / 64) * 8192 + k * 128) : (uint32_t)(row * 128);
+      const int at = MN ? row % 64 : k, sw = (MN ? k : row) & 7;
+      const uint32_t off = line + (uint32_t)(((at >> 3) ^ sw) << 4) + (uint32_t)(at & 7) * 2;
+      uint2 h, m, l;
+      split3(r[i].x, r[i].y, h.x, m.x, l.x);
+      split3(r[i].z, r[i].w, h.y, m.y, l.y);
+      *reinterpret_cast<uint2 *>(planes + off) = h;
+      *reinterpret_cast<uint2 *>(planes + PLANE + off) = m;
+      *reinterpret_cast<uint2 *>(planes + 2 * PLANE + off) = l;
+      const float big4 = fmaxf(fmaxf(fabsf(r[i].x), fabsf(r[i].y)), fmaxf(fabsf(r[i].z), fabsf(r[i].w)));
+      big |= big4 >= 1.7014118346046923e38f;   // 2^127; a NaN beside it does not hide it (fmaxf drops NaN)
+    }
+    return big;
+  }
+};
+
+__device__ __forceinline__ void f3_tile(const GemmF32TcArgs &g, int unit, int &z, int &split, int &mt, int &nt) {
+  const int per = g.tiles_m * g.tiles_n;
+  const int s = unit / per, r = unit - s * per;
+  split = s % g.splits;
+  z = s / g.splits;
+  constexpr int GROUP_M = 8;   // tiles that run together share operand rows in L2
+  const int group = r / (GROUP_M * g.tiles_n), first = group * GROUP_M;
+  const int gm = min(GROUP_M, g.tiles_m - first), in = r - first * g.tiles_n;
+  mt = first + in % gm;
+  nt = in / gm;
+}
+
+// the value that goes to C for accumulated sum v
+__device__ __forceinline__ float f3_finish(int epilogue, float v, float aux) {
+  if (epilogue == ALPHA_EPI_GELU) return gelu_f(v);
+  if (epilogue == ALPHA_EPI_ADD) return v + aux;
+  if (epilogue == ALPHA_EPI_GELU_BWD) return v * gelu_grad_f(aux);
+  return v;
+}
+
+template <bool A_MN, bool B_MN, int BN>
+__global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF32TcArgs g) {
+  using L = F3Layout<BN>;
+  extern __shared__ uint8_t f3_smem_raw[];
+  uint8_t *smem = (uint8_t *)(((uintptr_t)f3_smem_raw + 1023) & ~(uintptr_t)1023);
+  const uint32_t bar = smem_u32(smem) + L::BAR_OFF;
+  auto full_bar = [&](int s) { return bar + 8u * s; };
+  auto empty_bar = [&](int s) { return bar + 8u * (F3_STAGES + s); };
+  auto tfull_bar = [&](int s) { return bar + 8u * (2 * F3_STAGES + s); };
+  auto tempty_bar = [&](int s) { return bar + 8u * (2 * F3_STAGES + 2 + s); };
+  uint32_t *tmem_slot = (uint32_t *)(smem + L::BAR_OFF + 8 * (2 * F3_STAGES + 4));
+  volatile uint32_t *abort_flag = (volatile uint32_t *)(tmem_slot + 1);
+  volatile uint32_t *big_tag = (volatile uint32_t *)(tmem_slot + 2);   // [F3_FLAGS]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int MMA_WARP = F3_OP_WARPS;
+  constexpr uint32_t TMEM_COLS = 2 * BN;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < F3_STAGES; s++) {
+      mbar_init(full_bar(s), F3_OP_WARPS);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int s = 0; s < 2; s++) {
+      mbar_init(tfull_bar(s), 1);
+      mbar_init(tempty_bar(s), F3_ACC_WARPS);
+    }
+    *abort_flag = 0;
+    for (int i = 0; i < F3_FLAGS; i++) big_tag[i] = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  if (warp == MMA_WARP) {
+    tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  grid_dependency_trigger();
+  grid_dependency_wait();   // everything above touched only this SM
+  const uint32_t tmem_base = *tmem_slot;
+  const int units = g.tiles_m * g.tiles_n * g.splits * g.batch;
+
+  if (warp < F3_OP_WARPS) {
+    // ── operands: global -> registers -> three bf16 planes ────────────────────────────────
+    const int tid = threadIdx.x;
+    F3Operand<A_MN, F3_BM> a;
+    F3Operand<B_MN, BN> b;
+    int unit = blockIdx.x, z, split, mt, nt, kb = 0, kb1 = 0;
+    auto enter = [&]() {   // coordinates of `unit`
+      f3_tile(g, unit, z, split, mt, nt);
+      kb = split * g.kb_per_split;
+      kb1 = min(g.kblocks, kb + g.kb_per_split);
+    };
+    auto load_a = [&]() { a.load(g.A + z * g.batch_a, g.lda, mt * F3_BM, g.M, kb * F3_BK, g.K, g.vec_a, tid); };
+    auto load_b = [&]() { b.load(g.B + z * g.batch_b, g.ldb, nt * BN, g.N, kb * F3_BK, g.K, g.vec_b, tid); };
+    if (unit < units) {
+      enter();
+      load_a();
+      load_b();
+    }
+    int stage = 0;
+    uint32_t phase = 0, it = 0;   // it: tiles of this CTA so far
+    while (unit < units) {
+      if (!mbar_wait(empty_bar(stage), phase ^ 1, abort_flag)) break;
+      uint8_t *st = smem + stage * L::STAGE;
+      // split and store this step; each operand's registers then take the next step's loads
+      const uint32_t it_now = it;
+      if (++kb == kb1) {
+        unit += gridDim.x;
+        it++;
+        if (unit < units) enter();
+      }
+      bool big = a.store(st, tid);
+      if (unit < units) load_a();
+      big |= b.store(st + 3 * L::A_PLANE, tid);
+      if (unit < units) load_b();
+      if (big) big_tag[it_now % F3_FLAGS] = it_now + 1;
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full_bar(stage));
+      if (++stage == F3_STAGES) { stage = 0; phase ^= 1; }
+    }
+  } else {
+    // ── accumulation and epilogue: 32 rows (TMEM lane quadrant) x BN/2 columns per warp ───
+    constexpr int NC = BN / 2;
+    const int ew = warp - F3_OP_WARPS, quad = warp & 3, half = ew >> 2;
+    float *stg = reinterpret_cast<float *>(smem + L::EPI_OFF + ew * 4096);
+    int acc = 0;
+    uint32_t acc_phase = 0, it = 0;
+    bool ok = true;
+    auto steps_of = [&](int unit) {   // K steps of a unit of work
+      const int split = unit / (g.tiles_m * g.tiles_n) % g.splits;
+      return min(g.kblocks, (split + 1) * g.kb_per_split) - split * g.kb_per_split;
+    };
+    // MMAs of the next K step (warp 8 alone; control flow and descriptors are warp-uniform)
+    int i_unit = blockIdx.x, i_left = i_unit < units ? steps_of(i_unit) : 0, i_stage = 0, i_acc = 0;
+    uint32_t i_phase = 0, i_acc_phase = 0;
+    auto issue_next = [&]() -> bool {
+      if (i_left == 0) return true;
+      if (!mbar_wait(tempty_bar(i_acc), i_acc_phase ^ 1, abort_flag) || !mbar_wait(full_bar(i_stage), i_phase, abort_flag))
+        return false;
+      tc_fence_after();
+      constexpr uint32_t idesc = make_idesc_bf16(F3_BM, BN, A_MN, B_MN);
+      // smallest products first; plane 0 = h, 1 = m, 2 = l
+      constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+      const uint32_t a_s = smem_u32(smem) + i_stage * L::STAGE, b_s = a_s + 3 * L::A_PLANE;
+      const uint32_t d = tmem_base + i_acc * BN;
+      const uint64_t ad = A_MN ? make_smem_desc(a_s, 8192, 1024) : make_smem_desc(a_s, 16, 1024);
+      const uint64_t bd = B_MN ? make_smem_desc(b_s, 8192, 1024) : make_smem_desc(b_s, 16, 1024);
+      if (elect_one()) {
+#pragma unroll
+        for (int p = 0; p < 6; p++) {
+#pragma unroll
+          for (int k = 0; k < F3_BK / 16; k++)
+            mma_bf16_ss(d, ad + ((PA[p] * L::A_PLANE + k * (A_MN ? 2048 : 32)) >> 4),
+                        bd + ((PB[p] * L::B_PLANE + k * (B_MN ? 2048 : 32)) >> 4), idesc, (p | k) ? 1u : 0u);
+        }
+        mma_commit(empty_bar(i_stage));
+        mma_commit(tfull_bar(i_acc));
+      }
+      __syncwarp();
+      if (++i_stage == F3_STAGES) { i_stage = 0; i_phase ^= 1; }
+      i_acc ^= 1;
+      if (i_acc == 0) i_acc_phase ^= 1;
+      if (--i_left == 0) {
+        i_unit += gridDim.x;
+        if (i_unit < units) i_left = steps_of(i_unit);
+      }
+      return true;
+    };
+    if (ew == 0) ok = issue_next();
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x, it++) {
+      int z, split, mt, nt;
+      f3_tile(g, unit, z, split, mt, nt);
+      const int kb0 = split * g.kb_per_split, n_kb = min(g.kblocks, kb0 + g.kb_per_split) - kb0;
+      uint64_t sum[NC / 2];
+#pragma unroll
+      for (int j = 0; j < NC / 2; j++) sum[j] = 0;
+      for (int kb = 0; kb < n_kb; kb++) {
+        if (ew == 0 && !issue_next()) { ok = false; break; }
+        if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < NC; c += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_base + acc * BN + half * NC + c + ((uint32_t)(quad * 32) << 16), r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; j += 2)
+            sum[(c + j) / 2] = f2_add(sum[(c + j) / 2], f2_pack(__uint_as_float(r[j]), __uint_as_float(r[j + 1])));
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tempty_bar(acc));
+        acc ^= 1;
+        if (acc == 0) acc_phase ^= 1;
+      }
+      if (!ok) break;
+      const int m_base = mt * F3_BM + quad * 32, n_base = nt * BN + half * NC;
+      const bool big = big_tag[it % F3_FLAGS] == it + 1;
+      float *C = g.C + split * g.split_c + z * g.batch_c;
+      const float *aux_in = g.aux_in;
+      const bool aux_read = g.epilogue == ALPHA_EPI_ADD || g.epilogue == ALPHA_EPI_GELU_BWD;
+#pragma unroll
+      for (int c = 0; c < NC; c += 32) {
+        if (n_base + c >= g.N || m_base >= g.M) continue;   // warp-uniform
+        // this lane's row of the 32 x 32 block into the staging rows (16-byte chunks swizzled by row)
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          float4 v;
+          f2_unpack(sum[(c + q * 4) / 2], v.x, v.y);
+          f2_unpack(sum[(c + q * 4) / 2 + 1], v.z, v.w);
+          *reinterpret_cast<float4 *>(stg + lane * 32 + ((q ^ (lane & 7)) << 2)) = v;
+        }
+        __syncwarp();
+        // and out again, eight lanes to a row: 128-byte segments
+        const int q = lane & 7, n = n_base + c + q * 4;
+#pragma unroll 1
+        for (int rr = lane >> 3; rr < 32; rr += 4) {
+          const int64_t m = m_base + rr;
+          if (m >= g.M || n >= g.N) continue;
+          const float4 s4 = *reinterpret_cast<const float4 *>(stg + rr * 32 + ((q ^ (rr & 7)) << 2));
+          float v[4] = {s4.x, s4.y, s4.z, s4.w}, x[4] = {0.f, 0.f, 0.f, 0.f}, o[4] = {0.f, 0.f, 0.f, 0.f};
+          if (big) {
+            const int k_end = min(g.K, (kb0 + n_kb) * F3_BK);
+            const float *A = g.A + z * g.batch_a, *B = g.B + z * g.batch_b;
+#pragma unroll 1
+            for (int j = 0; j < 4; j++) {
+              const float had = j == 0 ? v[0] : j == 1 ? v[1] : j == 2 ? v[2] : v[3];
+              if (n + j >= g.N || isfinite(had)) continue;
+              float t = 0.f;
+              for (int k = kb0 * F3_BK; k < k_end; k++)
+                t = fmaf(A_MN ? A[k * g.lda + m] : A[m * g.lda + k], B_MN ? B[k * g.ldb + n + j] : B[(n + j) * g.ldb + k], t);
+              if (j == 0) v[0] = t; else if (j == 1) v[1] = t; else if (j == 2) v[2] = t; else v[3] = t;
+            }
+          }
+          float *dst = C + m * g.ldc + n;
+          const int64_t aux_at = m * g.ld_aux + n;
+          if (g.vec_c && n + 4 <= g.N) {
+            if (aux_read) {
+              const float4 t = *reinterpret_cast<const float4 *>(aux_in + aux_at);
+              x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+            }
+            if (g.accumulate) {
+              const float4 t = *reinterpret_cast<const float4 *>(dst);
+              o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
+            }
+            if (g.epilogue == ALPHA_EPI_GELU) *reinterpret_cast<float4 *>(g.aux_out + aux_at) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              v[j] = f3_finish(g.epilogue, v[j], x[j]);
+              if (g.accumulate) v[j] = o[j] + v[j];
+            }
+            *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              if (n + j >= g.N) continue;
+              if (g.epilogue == ALPHA_EPI_GELU) g.aux_out[aux_at + j] = v[j];
+              const float y = f3_finish(g.epilogue, v[j], aux_read ? aux_in[aux_at + j] : 0.f);
+              dst[j] = g.accumulate ? dst[j] + y : y;
+            }
+          }
+        }
+        __syncwarp();   // the staging rows are overwritten by the next block
+      }
+    }
+  }
+
+  if (*abort_flag) {
+    // a wait ran out: MMAs in flight get time to finish before shared memory is released, then report
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000ll) {
+    }
+    if (threadIdx.x == 0 && g.err) atomicExch(g.err, 0x6D000000u | (uint32_t)(blockIdx.x & 0xFFFF));
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == MMA_WARP) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
+// C = finish(sum of the slabs in split order)
+__global__ void __launch_bounds__(256) gemm_f32_reduce_kernel(const GemmF32TcArgs g, const float *__restrict__ ws,
+                                                              float *C, int64_t ldc, int64_t batch_c, int epilogue,
+                                                              int accumulate, int vec) {
+  grid_dependency_trigger();
+  grid_dependency_wait();   // the slabs come from the kernel launched just before
+  const int64_t mn = (int64_t)g.M * g.N, total = mn * g.batch;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x * (vec ? 4 : 1);
+  for (int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * (vec ? 4 : 1); e < total; e += step) {
+    const int64_t z = e / mn, r = e - z * mn, m = r / g.N, n = r - m * g.N;
+    float *dst = C + z * batch_c + m * ldc + n;
+    const int64_t aux_at = m * g.ld_aux + n;
+    if (vec) {
+      float4 s = *reinterpret_cast<const float4 *>(ws + e);
+#pragma unroll 4
+      for (int k = 1; k < g.splits; k++) {
+        const float4 t = *reinterpret_cast<const float4 *>(ws + (int64_t)k * g.split_c + e);
+        s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+      }
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (epilogue == ALPHA_EPI_ADD || epilogue == ALPHA_EPI_GELU_BWD) x = *reinterpret_cast<const float4 *>(g.aux_in + aux_at);
+      if (epilogue == ALPHA_EPI_GELU) *reinterpret_cast<float4 *>(g.aux_out + aux_at) = s;
+      s = make_float4(f3_finish(epilogue, s.x, x.x), f3_finish(epilogue, s.y, x.y), f3_finish(epilogue, s.z, x.z),
+                      f3_finish(epilogue, s.w, x.w));
+      if (accumulate) {
+        const float4 o = *reinterpret_cast<const float4 *>(dst);
+        s.x = o.x + s.x; s.y = o.y + s.y; s.z = o.z + s.z; s.w = o.w + s.w;
+      }
+      *reinterpret_cast<float4 *>(dst) = s;
+    } else {
+      float s = 0.f;
+      for (int k = 0; k < g.splits; k++) s += ws[(int64_t)k * g.split_c + e];
+      if (epilogue == ALPHA_EPI_GELU) g.aux_out[aux_at] = s;
+      s = f3_finish(epilogue, s, epilogue == ALPHA_EPI_ADD || epilogue == ALPHA_EPI_GELU_BWD ? g.aux_in[aux_at] : 0.f);
+      *dst = accumulate ? *dst + s : s;
+    }
+  }
+}
+
+template <bool A_MN, bool B_MN, int BN>
+static int f3_launch(const GemmF32TcArgs &g, int grid) {
+  static int attr = -1;
+  if (attr != g_init_epoch) {
+    ALPHA_CUDA(cudaFuncSetAttribute(gemm_f32_tc_kernel<A_MN, B_MN, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    F3Layout<BN>::DYN));
+    attr = g_init_epoch;
+  }
+  ALPHA_CUDA(launch_overlapped(OVL_GEMM, gemm_f32_tc_kernel<A_MN, B_MN, BN>, dim3(grid), dim3(F3_THREADS),
+                               F3Layout<BN>::DYN, g));
+  ALPHA_LAUNCHED();
+  return 0;
+}
+
+// Tile width and number of K splits: the pair that minimises waves x (K steps + fixed part) plus the
+// pass that adds the splits, in cycles of one SM.
+static void f3_plan(int64_t M, int64_t N, int64_t kblocks, int64_t batch, int &bn, int &splits) {
+  double best = 1e300;
+  for (int w = 128; w >= 64; w -= 64) {
+    const int64_t tiles = ((M + F3_BM - 1) / F3_BM) * ((N + w - 1) / w) * batch;
+    const double per_kb = w == 128 ? 2300.0 : 1500.0, fixed = 4000.0;
+    for (int64_t sp = 1; sp <= kblocks && sp <= 64; sp++) {
+      const int64_t waves = (tiles * sp + g_sm_count - 1) / g_sm_count, kb = (kblocks + sp - 1) / sp;
+      double t = (double)waves * (double)kb * per_kb + fixed;
+      if (sp > 1) t += 4000.0 + (double)(2 * sp + 1) * (double)M * (double)N * (double)batch * 4.0 / 2700.0;
+      if (t < best) {
+        best = t;
+        bn = w;
+        splits = (int)sp;
+      }
+    }
+  }
+}
+
+int gemm_f32_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M, int64_t N, int64_t K, int64_t lda,
+                       int64_t ldb, int64_t ldc, int epilogue, alpha_buf aux, int64_t ld_aux, int accumulate,
+                       int64_t batch, int64_t stride_a, int64_t stride_b, int64_t stride_c) {
+  const bool a_mn = layout == ALPHA_GEMM_TN, b_mn = layout != ALPHA_GEMM_NT;
+  GemmF32TcArgs g;
+  memset(&g, 0, sizeof(g));
+  g.A = ptr<float>(A); g.B = ptr<float>(B); g.C = ptr<float>(C);
+  g.aux_in = ptr<float>(aux); g.aux_out = ptr<float>(aux);
+  g.lda = lda; g.ldb = ldb; g.ldc = ldc; g.ld_aux = ld_aux;
+  g.batch_a = stride_a; g.batch_b = stride_b; g.batch_c = stride_c;
+  g.M = (int)M; g.N = (int)N; g.K = (int)K; g.batch = (int)batch;
+  g.kblocks = (int)((K + F3_BK - 1) / F3_BK);
+  int bn = 128, splits = 1;
+  f3_plan(M, N, g.kblocks, batch, bn, splits);
+  g.kb_per_split = (g.kblocks + splits - 1) / splits;
+  g.splits = splits = (g.kblocks + g.kb_per_split - 1) / g.kb_per_split;   // drop empty splits
+  g.tiles_m = (int)((M + F3_BM - 1) / F3_BM);
+  g.tiles_n = (int)((N + bn - 1) / bn);
+  g.epilogue = epilogue; g.accumulate = accumulate;
+  auto vec = [&](alpha_buf p, int64_t ld, int64_t stride) {
+    return (p & 15) == 0 && ld % 4 == 0 && (batch == 1 || stride % 4 == 0);
+  };
+  g.vec_a = vec(A, lda, stride_a);
+  g.vec_b = vec(B, ldb, stride_b);
+  const bool aux_vec = epilogue == ALPHA_EPI_NONE || ((aux & 15) == 0 && ld_aux % 4 == 0);
+  const bool out_vec = vec(C, ldc, stride_c) && aux_vec;
+  g.vec_c = out_vec;
+  g.err = tc_error_word();
+  void *ws = nullptr;
+  if (splits > 1) {
+    g.split_c = batch * M * N;
+    if (pool_alloc((size_t)splits * g.split_c * sizeof(float), &ws)) return 1;
+    g.C = (float *)ws; g.ldc = N; g.batch_c = M * N;
+    g.epilogue = ALPHA_EPI_NONE; g.accumulate = 0;
+    g.vec_c = N % 4 == 0;
+  }
+  const int64_t units = (int64_t)g.tiles_m * g.tiles_n * splits * batch;
+  const int grid = (int)(units < g_sm_count ? units : g_sm_count);
+  int rc;
+  if (bn == 128)
+    rc = a_mn ? f3_launch<true, true, 128>(g, grid) : b_mn ? f3_launch<false, true, 128>(g, grid) : f3_launch<false, false, 128>(g, grid);
+  else
+    rc = a_mn ? f3_launch<true, true, 64>(g, grid) : b_mn ? f3_launch<false, true, 64>(g, grid) : f3_launch<false, false, 64>(g, grid);
+  if (rc == 0 && splits > 1) {
+    const int v = out_vec && N % 4 == 0;
+    const cudaError_t e = launch_overlapped(OVL_SPLITK, gemm_f32_reduce_kernel,
+                                            dim3(grid_for(batch * M * N / (v ? 4 : 1) + 1, 256, 8)), dim3(256), 0, g,
+                                            (const float *)ws, ptr<float>(C), ldc, stride_c, epilogue, accumulate, v);
+    if (e != cudaSuccess) rc = set_error("alpha_gemm: reduce launch -> %s", cudaGetErrorString(e));
+    else g_launches++;
+  }
+  if (ws) pool_free(ws);
+  return rc;
+}
+
+}  // namespace alpha

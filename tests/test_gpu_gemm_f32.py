@@ -1,0 +1,147 @@
+"""The fp32 GEMM (bf16-triple products on the tensor cores) against numpy in 64 bits.
+
+The bound: with u = 2^-24, a dot product that sums K rounded terms in chains no longer than n has a
+forward error of at most about n*u*sum|a||b|; chains here are 64 (inside a K step, truncating: 2u per
+add) and K/64 (between them).  The operand splits add 3u.  So every element must be within
+(2*(64/16*6) + K/64 + 8)*u*(|A| @ |B|), which for K = 256 is a quarter of an FMA loop's own bound.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -24
+
+
+@pytest.fixture(scope="module")
+def B():
+    from alpha2_b200.backend import CudaBackend
+    b = CudaBackend(0)
+    yield b
+    b.checkAsyncError()
+
+
+def bound(a, b, K):
+    return (48 + K / 64 + 8) * U * (np.abs(a) @ np.abs(b))
+
+
+def product(B, layout, a, b, M, N, K, lda=None, ldb=None, epilogue=0, aux=None, accumulate=0, c0=None):
+    """C of alpha_gemm; a, b are the arrays as stored, rows padded with 7s to the leading dimension."""
+    from alpha2_b200 import _lib as L
+    from alpha2_b200._lib import check
+
+    def up(x, ld):
+        if ld and ld > x.shape[1]:
+            x = np.concatenate([x, np.full((x.shape[0], ld - x.shape[1]), 7, np.float32)], 1)
+        return B.upload(np.ascontiguousarray(x, np.float32), "f32")
+
+    A, Bm = up(a, lda), up(b, ldb)
+    C = B.upload(np.zeros((M, N), np.float32) if c0 is None else c0, "f32")
+    check(B.lib.alpha_gemm(layout, A.ptr, Bm.ptr, C.ptr, M, N, K, lda or a.shape[1], ldb or b.shape[1], N, L.F32, L.F32,
+                           epilogue, aux.ptr if aux is not None else 0, N, accumulate))
+    C.invalidate_host()
+    return np.array(C.data, np.float64).reshape(M, N)
+
+
+def operands(layout, M, N, K, seed, scale=1.0):
+    g = np.random.default_rng(seed)
+    a, b = (g.standard_normal((M, K)) * scale).astype(np.float32), g.standard_normal((K, N)).astype(np.float32)
+    stored = {0: (a, b.T), 1: (a, b), 2: (a.T, b)}[layout]
+    return a.astype(np.float64), b.astype(np.float64), stored
+
+
+# edges of the 128 x {64, 128} x 64 tiles, one short and one over, both tile widths, one and many splits
+@pytest.mark.parametrize("layout", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 64, 64), (3, 5, 7), (127, 65, 63), (128, 128, 64), (129, 129, 65),
+                                   (256, 192, 64), (48, 1152, 384), (200, 96, 1536), (257, 512, 130),
+                                   (1024, 1024, 256), (96, 64, 16384), (4096, 72, 100), (2500, 1300, 40)])
+def test_against_64_bits(B, layout, M, N, K):
+    a, b, (sa, sb) = operands(layout, M, N, K, M + N + K)
+    got = product(B, layout, sa, sb, M, N, K)
+    assert np.all(np.abs(got - a @ b) <= bound(a, b, K))
+
+
+@pytest.mark.parametrize("layout", [0, 1, 2])
+@pytest.mark.parametrize("pad", [1, 4])      # 16-byte rows lost and kept
+def test_padded_rows(B, layout, pad):
+    M, N, K = 130, 70, 100
+    a, b, (sa, sb) = operands(layout, M, N, K, pad)
+    got = product(B, layout, sa, sb, M, N, K, sa.shape[1] + pad, sb.shape[1] + pad)
+    assert np.all(np.abs(got - a @ b) <= bound(a, b, K))
+
+
+@pytest.mark.parametrize("M,N,K", [(130, 66, 64), (64, 136, 2048)])    # one split; split over K
+@pytest.mark.parametrize("epilogue", [0, 1, 2, 3])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_epilogues(B, M, N, K, epilogue, accumulate):
+    a, b, (sa, sb) = operands(0, M, N, K, epilogue, 0.05)
+    g = np.random.default_rng(9)
+    x, c0 = (g.standard_normal((M, N)).astype(np.float32) for _ in range(2))
+    aux = B.upload(x, "f32")
+    got = product(B, 0, sa, sb, M, N, K, epilogue=epilogue, aux=aux, accumulate=accumulate, c0=c0)
+    r, x = a @ b, x.astype(np.float64)
+    err = bound(a, b, K)
+    gelu = lambda t: 0.5 * t * (1 + np.tanh(0.7978845608028654 * (t + 0.044715 * t ** 3)))
+    th = np.tanh(0.7978845608028654 * (x + 0.044715 * x ** 3))
+    slope = 0.5 * (1 + th) + 0.5 * x * (1 - th ** 2) * 0.7978845608028654 * (1 + 3 * 0.044715 * x ** 2)
+    want = [r, gelu(r), r + x, r * slope][epilogue] + accumulate * c0
+    if epilogue == 1:
+        aux.invalidate_host()
+        assert np.all(np.abs(np.array(aux.data, np.float64) - r) <= err)    # the pre-activation
+    # |gelu'| < 1.13; the epilogue's own arithmetic: a dozen roundings of values up to this size
+    assert np.all(np.abs(got - want) <= 1.13 * err + 16 * U * (np.abs(want) + np.abs(x) + np.abs(r) + np.abs(c0)))
+
+
+@pytest.mark.parametrize("layout", [0, 1, 2])
+@pytest.mark.parametrize("K", [100, 2048])
+def test_infinities_and_huge_values(B, layout, K):
+    """inf * finite, inf * 0, values that round to inf in 16 bits and NaN: as an fmaf chain gives them."""
+    M, N = 140, 70
+    a, b, _ = operands(1, M, N, K, 3)
+    a[5, 9], a[6, 10], a[131, 3], a[7, 1] = np.inf, -np.inf, 3.4e38, np.nan
+    b[:, 2] = np.where(np.arange(K) % 2, 0.0, b[:, 2])
+    b[9, 4], b[3, :] = 0.0, 0.25
+    a, b = (x.astype(np.float32).astype(np.float64) for x in (a, b))
+    stored = {0: (a, b.T), 1: (a, b), 2: (a.T, b)}[layout]
+    got = product(B, layout, *stored, M, N, K)
+    with np.errstate(invalid="ignore"):
+        want = a @ b
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    fin = np.isfinite(want)
+    finite = lambda x: np.where(np.isfinite(x), x, 0.0)
+    # the recomputed elements are a chain of K
+    assert np.all(np.abs(got - want)[fin] <= (bound(finite(a), b, K) + K * U * (np.abs(finite(a)) @ np.abs(b)))[fin])
+
+
+@pytest.mark.parametrize("exponent", [-100, -30, 30, 100])
+def test_scales(B, exponent):
+    """Products far from 1: the lowest term of a split stays representable down to operands of 2^-100."""
+    M, N, K = 128, 64, 128
+    a, b, _ = operands(1, M, N, K, 5)
+    a = (a * 2.0 ** exponent).astype(np.float32).astype(np.float64)
+    got = product(B, 1, a, b, M, N, K)
+    assert np.all(np.abs(got - a @ b) <= bound(a, b, K))
+
+
+@pytest.mark.parametrize("nb", [1, 5])
+@pytest.mark.parametrize("layout", [0, 1, 2])
+def test_batched(B, nb, layout):
+    from alpha2_b200._lib import check
+    M, N, K = 70, 33, 96
+    a, b = (np.stack(x) for x in zip(*(operands(layout, M, N, K, i)[:2] for i in range(nb))))
+    sa, sb = (a.transpose(0, 2, 1) if layout == 2 else a), (b.transpose(0, 2, 1) if layout == 0 else b)
+    A, Bm = (B.upload(np.ascontiguousarray(x, np.float32), "f32") for x in (sa, sb))
+    C = B.zeros((nb, M, N), "f32")
+    check(B.lib.alpha_gemm_batched_f32(layout, A.ptr, Bm.ptr, C.ptr, M, N, K, sa.shape[2], sb.shape[2], N, nb, M * K,
+                                       K * N, M * N))
+    got = np.array(C.data, np.float64)
+    for i in range(nb):
+        assert np.all(np.abs(got[i] - a[i] @ b[i]) <= bound(a[i], b[i], K))
+
+
+def test_same_bits_every_time(B):
+    M, N, K = 700, 260, 4000
+    _, _, (sa, sb) = operands(2, M, N, K, 1)
+    first = product(B, 2, sa, sb, M, N, K)
+    assert all(np.array_equal(first, product(B, 2, sa, sb, M, N, K)) for _ in range(5))
