@@ -1,7 +1,7 @@
 // Entry points of the fused attention (Backend.flashAttention / flashAttentionBackward,
 // packages/core/src/interfaces.ts:127-135): pick the kernel family for the storage type.
-// bf16 with head dim 64 runs on the tensor cores (attn_tc.cu); everything else — fp32
-// storage (the parity mode) and other head sizes — runs the fp32 FMA kernels (attn_f32.cu).
+// bf16 with head dim 64 runs on tcgen05 (attn_tc.cu); everything else — fp32 storage (the
+// parity mode) and other head sizes — runs the fp32-accurate kernels of attn_f32.cu.
 #include "common.cuh"
 
 namespace alpha {

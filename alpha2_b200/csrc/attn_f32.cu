@@ -1,6 +1,6 @@
-// Causal flash attention, forward and backward, with fp32 arithmetic on the FMA pipes.
-// This is the full-precision mode (fp32 parity configurations) and it accepts bf16
-// storage too; the tensor-core kernels for bf16 live in attn_tc.cu.
+// Causal flash attention, forward and backward, in fp32 accuracy on the tensor cores: fp32 storage
+// (any of the head sizes 16 / 32 / 64 / 128) and bf16 storage of the head sizes that attn_tc.cu does
+// not take.
 //
 // Contract: Backend.flashAttention / flashAttentionBackward
 // (packages/core/src/interfaces.ts:127-135).  Math as in the reference kernels
@@ -11,15 +11,35 @@
 //
 // q/k/v/o are addressed through (batch, head, time) element strides so the kernel reads
 // the fused QKV projection in place and writes O already head-merged; nothing is
-// transposed or copied around it.  Tiles are 64 queries x 64 keys; 256 threads as a 16x16
-// grid, each owning a 4x4 patch of the score tile and a 4 x (D/16) patch of the outputs.
-// dK/dV and dQ are separate kernels (each output tile has one owner, no atomics, so the
-// gradients are deterministic).
-#include "common.cuh"
+// transposed or copied around it.
+//
+// Every fp32 number that enters a product — q, k, v, dO from memory, P and dS from registers — is
+// held as three bf16 terms (x = h + m + l, all 24 bits), and a product is the sum of the six term
+// products of weight 2^-16 and above; bf16 storage is one term.  The tensor core adds truncating, so
+// it never sees a long sum: scores are one chain over D, small terms first, and the contribution
+// of 32 or 64 keys (queries) to an output is summed on its own and then added in fp32
+// registers, round to nearest.
+//
+// Warp-level mma.sync rather than tcgen05: P and dS are produced in registers in the layout that
+// the next product wants its left operand in, so the three-term splits never leave the register file
+// (through shared memory they would be 6 bytes out and 6 bytes in per score and product).
+// Tiles are 64 queries x 64 keys, four warps with 16 rows each.  dK/dV and dQ are separate
+// kernels (each output tile has one owner, no atomics, so the gradients are deterministic).
+//
+// Measured on a B200, forward / dK+dV / dQ per layer against FMA-pipe kernels of the same tiling: 512 heads,
+// T 256, D 32, fp32: 122 / 190 / 225 us (167 / 315 / 217); bf16 storage, 256 heads: 59 / 54 / 68 (97 / 161 /
+// 113); the dQ times include its wait for the dK/dV kernel that it overlaps.  Bound by the score arithmetic
+// (accurate tanh and exp, the splits) and by two to three blocks an SM to hide its latency.
+#include <string.h>
+
+#include "tc_common.cuh"
 
 namespace alpha {
 
-constexpr int BQ = 64, BKV = 64, PAD = 4;
+using tc::bf16x2_pack;
+using tc::smem_u32;
+
+constexpr int BQ = 64, BKV = 64, ATTN_THREADS = 128;
 
 struct AttnArgs {
   const void *q, *k, *v, *o, *d_o;
@@ -30,150 +50,318 @@ struct AttnArgs {
   int64_t q_sb, q_sh, q_st, o_sb, o_sh, o_st;
   int H, T;
   float scale, cap;
+  float cap_arg;      // scale / cap: the argument of tanh per raw score
+  int vec_q, vec_o;   // four consecutive elements of q/k/v and their gradients / of o and dO can move at once
 };
 
-// global [rows x D] (row stride st) -> shared row-major [64][D+PAD], zero-filled past T
+template <typename T> struct Terms { static constexpr int N = 3; };
+template <> struct Terms<__nv_bfloat16> { static constexpr int N = 1; };
+
+// Shared-memory tile of 64 rows x D: one bf16 plane per term, rows 16 bytes longer than their data so
+// that the eight rows of an ldmatrix fall into different banks.
 template <typename T, int D>
-__device__ __forceinline__ void load_rows(float *dst, const T *src, int64_t st, int t0, int Tlen) {
-  for (int e = threadIdx.x; e < 64 * D; e += 256) {
-    const int r = e / D, c = e - r * D;
-    const int t = t0 + r;
-    dst[r * (D + PAD) + c] = t < Tlen ? to_f32(src[(int64_t)t * st + c]) : 0.f;
-  }
+struct AttnTile {
+  static constexpr int NT = Terms<T>::N, PITCH = 2 * D + 16, PLANE = 64 * PITCH, BYTES = NT * PLANE;
+};
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
 }
-// global [rows x D] -> shared transposed [D][64+PAD]
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+// c[16x8] += a[16x16] b[16x8]
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// a pair of fp32 numbers as three pairs of bf16 terms
+__device__ __forceinline__ void terms3(float x0, float x1, uint32_t &h, uint32_t &m, uint32_t &l) {
+  h = bf16x2_pack(x0, x1);
+  const float r0 = x0 - __uint_as_float(h << 16), r1 = x1 - __uint_as_float(h & 0xFFFF0000u);
+  m = bf16x2_pack(r0, r1);
+  l = bf16x2_pack(r0 - __uint_as_float(m << 16), r1 - __uint_as_float(m & 0xFFFF0000u));
+}
+
+// Global rows [t0, t0 + 64) x D (row stride st) -> the planes of a tile, zeros past Tlen.  Returns whether
+// the thread saw an infinity or a value from 2^127 on (which may round to one): see fix_scores.
 template <typename T, int D>
-__device__ __forceinline__ void load_rows_t(float *dst, const T *src, int64_t st, int t0, int Tlen) {
-  for (int e = threadIdx.x; e < 64 * D; e += 256) {
-    const int r = e / D, c = e - r * D;
-    const int t = t0 + r;
-    dst[c * (64 + PAD) + r] = t < Tlen ? to_f32(src[(int64_t)t * st + c]) : 0.f;
+__device__ __forceinline__ bool load_tile(uint8_t *dst, const T *src, int64_t st, int t0, int Tlen, int vec) {
+  using L = AttnTile<T, D>;
+  bool big = false;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < 64 * D / 4; e += ATTN_THREADS) {
+    const int r = e / (D / 4), c = (e % (D / 4)) * 4, t = t0 + r;
+    uint8_t *at = dst + r * L::PITCH + c * 2;
+    const T *p = src + (int64_t)t * st + c;
+    if constexpr (sizeof(T) == 2) {
+      uint2 x = make_uint2(0, 0);
+      if (t < Tlen) {
+        if (vec) {
+          x = *reinterpret_cast<const uint2 *>(p);
+        } else {
+          const uint16_t *u = reinterpret_cast<const uint16_t *>(p);
+          x = make_uint2(u[0] | ((uint32_t)u[1] << 16), u[2] | ((uint32_t)u[3] << 16));
+        }
+      }
+      *reinterpret_cast<uint2 *>(at) = x;
+    } else {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < Tlen) {
+        if (vec) x = *reinterpret_cast<const float4 *>(p);
+        else x = make_float4(p[0], p[1], p[2], p[3]);
+      }
+      uint2 h, m, l;
+      terms3(x.x, x.y, h.x, m.x, l.x);
+      terms3(x.z, x.w, h.y, m.y, l.y);
+      *reinterpret_cast<uint2 *>(at) = h;
+      *reinterpret_cast<uint2 *>(at + L::PLANE) = m;
+      *reinterpret_cast<uint2 *>(at + 2 * L::PLANE) = l;
+      big |= fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))) >= 1.7014118346046923e38f;
+    }
+  }
+  return big;
+}
+
+// acc[n] = A B^T for the warp's 16 rows of tile A and the 8 * NN rows of tile B from row b0 on.  Pairs of
+// 8-row groups [from, to) are computed, the others stay zero (causal skipping, warp-uniform).
+template <typename T, int D, int NN>
+__device__ __forceinline__ void score_product(float (&acc)[NN][4], uint32_t a_tile, int a_row, uint32_t b_tile, int b0,
+                                              int from, int to, int lane) {
+  using L = AttnTile<T, D>;
+  const uint32_t a_at = a_tile + (a_row + (lane & 15)) * L::PITCH + (lane >> 4) * 16;
+  const uint32_t b_at = b_tile + (b0 + ((lane >> 4) & 1) * 8 + (lane & 7)) * L::PITCH + ((lane >> 3) & 1) * 16;
+#pragma unroll
+  for (int n = 0; n < NN; n++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) acc[n][i] = 0.f;
+  if constexpr (L::NT == 3) {
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ks++) {
+      uint32_t a[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; i++) ldsm4(a[i], a_at + i * L::PLANE + ks * 32);
+#pragma unroll
+      for (int p = 0; p < NN / 2; p++) {
+        if (p < from || p >= to) continue;
+        uint32_t b[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; i++) ldsm4(b[i], b_at + i * L::PLANE + p * 16 * L::PITCH + ks * 32);
+#pragma unroll
+        for (int w = 2; w >= 1; w--)
+#pragma unroll
+          for (int i = 0; i <= w; i++) {
+            mma16816(acc[2 * p], a[i], b[w - i][0], b[w - i][1]);
+            mma16816(acc[2 * p + 1], a[i], b[w - i][2], b[w - i][3]);
+          }
+      }
+    }
+  }
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ks++) {
+    uint32_t a[4];
+    ldsm4(a, a_at + ks * 32);
+#pragma unroll
+    for (int p = 0; p < NN / 2; p++) {
+      if (p < from || p >= to) continue;
+      uint32_t b[4];
+      ldsm4(b, b_at + p * 16 * L::PITCH + ks * 32);
+      mma16816(acc[2 * p], a, b[0], b[1]);
+      mma16816(acc[2 * p + 1], a, b[2], b[3]);
+    }
   }
 }
 
-// acc[i][j] = sum_d A[ty*4+i][d] * Bt[d][tx*4+j]   (A row-major [64][D+PAD], Bt [D][64+PAD])
-template <int D>
-__device__ __forceinline__ void tile_abt(float (&acc)[4][4], const float *A, const float *Bt, int ty, int tx) {
+// Left operand of an output product: the accumulator of 2 * KS 8-column groups as three bf16 terms in
+// the register layout of A.
+template <int KS>
+struct LeftTerms {
+  uint32_t t[3][KS][4];
+  __device__ __forceinline__ void set(const float (&x)[2 * KS][4]) {
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+    for (int k = 0; k < KS; k++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-#pragma unroll 8
-  for (int d = 0; d < D; d++) {
-    const float4 b4 = *reinterpret_cast<const float4 *>(&Bt[d * (64 + PAD) + tx * 4]);
-    const float b[4] = {b4.x, b4.y, b4.z, b4.w};
+      for (int i = 0; i < 4; i++)   // a0: rows 0-7, columns 0-7; a1: rows 8-15; a2, a3: columns 8-15
+        terms3(x[2 * k + (i >> 1)][(i & 1) * 2], x[2 * k + (i >> 1)][(i & 1) * 2 + 1], t[0][k][i], t[1][k][i], t[2][k][i]);
+  }
+};
+
+// out[n] = out[n] * f + (A B)[n] for the warp's 16 rows: A from registers (16 x 16*KS), B rows b0.. of a tile,
+// 8-column groups n of D.  Steps [from, to) of 16 rows of B are used.
+template <typename T, int D, int KS, bool RESCALE>
+__device__ __forceinline__ void output_product(float (&out)[D / 8][4], const LeftTerms<KS> &a, uint32_t b_tile, int b0,
+                                               int from, int to, float f0, float f1, int lane) {
+  using L = AttnTile<T, D>;
+  constexpr int G = D >= 32 ? 2 : 1;   // pairs of column groups at a time: independent chains
+  const uint32_t b_at = b_tile + (b0 + ((lane >> 3) & 1) * 8 + (lane & 7)) * L::PITCH + ((lane >> 4) & 1) * 16;
+#pragma unroll
+  for (int g = 0; g < D / 16; g += G) {
+    float t[2 * G][4];
+#pragma unroll
+    for (int n = 0; n < 2 * G; n++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) t[n][i] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KS; k++) {
+      if (k < from || k >= to) continue;
+      uint32_t b[G][L::NT][4];
+#pragma unroll
+      for (int p = 0; p < G; p++)
+#pragma unroll
+        for (int j = 0; j < L::NT; j++) ldsm4_t(b[p][j], b_at + j * L::PLANE + k * 16 * L::PITCH + (g + p) * 32);
+#pragma unroll
+      for (int w = 2; w >= 1; w--)
+#pragma unroll
+        for (int j = 0; j <= w; j++) {
+          if (j >= L::NT) continue;
+#pragma unroll
+          for (int p = 0; p < G; p++) {
+            mma16816(t[2 * p], a.t[w - j][k], b[p][j][0], b[p][j][1]);
+            mma16816(t[2 * p + 1], a.t[w - j][k], b[p][j][2], b[p][j][3]);
+          }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < KS; k++) {
+      if (k < from || k >= to) continue;
+#pragma unroll
+      for (int p = 0; p < G; p++) {
+        uint32_t b[4];
+        ldsm4_t(b, b_at + k * 16 * L::PITCH + (g + p) * 32);
+        mma16816(t[2 * p], a.t[0][k], b[0], b[1]);
+        mma16816(t[2 * p + 1], a.t[0][k], b[2], b[3]);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 2 * G; n++)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        out[2 * g + n][i] = RESCALE ? fmaf(out[2 * g + n][i], i < 2 ? f0 : f1, t[n][i]) : out[2 * g + n][i] + t[n][i];
+  }
+}
+
+// Scores that came out non-finite in a tile that holds an infinity (inf has no split: inf = inf + NaN) or
+// a value that rounds to one: an fmaf chain over D instead, so that inf * x stays an infinity, which the
+// soft cap maps to the cap.  Infinities in v or dO, which meet P and dS, turn what they reach into NaN.
+template <typename T, int D>
+__device__ __noinline__ float score_fma(const T *a, const T *b) {
+  float s = 0.f;
+#pragma unroll 1
+  for (int d = 0; d < D; d++) s = fmaf(to_f32(a[d]), to_f32(b[d]), s);
+  return s;
+}
+template <typename T, int D, int NN>
+__device__ __forceinline__ void fix_scores(float (&acc)[NN][4], const T *a, const T *b, int64_t a_st, int64_t b_st, int ar,
+                                           int br, int Tlen) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int n = 0; n < NN; n++)
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      const float a = A[(ty * 4 + i) * (D + PAD) + d];
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a, b[j], acc[i][j]);
+      const int r = ar + lane / 4 + (i >> 1) * 8, c = br + n * 8 + (lane & 3) * 2 + (i & 1);
+      if (!isfinite(acc[n][i]) && r < Tlen && c < Tlen)
+        acc[n][i] = score_fma<T, D>(a + (int64_t)r * a_st, b + (int64_t)c * b_st);
     }
-  }
 }
 
-// out[i][j] += sum_r W[r][ty*4+i] * X[r][tx*CPT+j]  (W [64][64+PAD] indexed [r][row], X row-major)
-template <int D, bool W_TRANSPOSED>
-__device__ __forceinline__ void tile_wx(float (&out)[4][D / 16], const float *W, const float *X, int ty, int tx) {
-  constexpr int CPT = D / 16;
-#pragma unroll 4
-  for (int r = 0; r < 64; r++) {
-    float w[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-      w[i] = W_TRANSPOSED ? W[r * (64 + PAD) + ty * 4 + i] : W[(ty * 4 + i) * (64 + PAD) + r];
-#pragma unroll
-    for (int j = 0; j < CPT; j++) {
-      const float x = X[r * (D + PAD) + tx * CPT + j];
-#pragma unroll
-      for (int i = 0; i < 4; i++) out[i][j] = fmaf(w[i], x, out[i][j]);
-    }
-  }
+// Four lanes of a quad share a row.
+__device__ __forceinline__ float quad_max(float v) {
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+  return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+__device__ __forceinline__ float quad_sum(float v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-__device__ __forceinline__ float half_warp_max(float v) {
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-__device__ __forceinline__ float half_warp_sum(float v) {
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+template <typename T>
+__device__ __forceinline__ void store_pair(T *p, float x, float y, int vec) {
+  if constexpr (sizeof(T) == 4) {
+    if (vec) { *reinterpret_cast<float2 *>(p) = make_float2(x, y); return; }
+  } else {
+    if (vec) { *reinterpret_cast<uint32_t *>(p) = bf16x2_pack(x, y); return; }
+  }
+  p[0] = from_f32<T>(x);
+  p[1] = from_f32<T>(y);
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(256) attn_fwd_kernel(AttnArgs a) {
-  extern __shared__ __align__(16) float sm[];
-  constexpr int CPT = D / 16;
-  float *Qs = sm;                          // [64][D+PAD]
-  float *Kt = Qs + 64 * (D + PAD);         // [D][64+PAD]
-  float *Vs = Kt + D * (64 + PAD);         // [64][D+PAD]
-  float *Ps = Vs + 64 * (D + PAD);         // [64][64+PAD]
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int qb = blockIdx.x, bh = blockIdx.y;
+__global__ void __launch_bounds__(ATTN_THREADS) attn_fwd_kernel(const AttnArgs a) {
+  using L = AttnTile<T, D>;
+  extern __shared__ __align__(16) uint8_t at_sm[];
+  uint8_t *Qs = at_sm, *Ks = Qs + L::BYTES, *Vs = Ks + L::BYTES;
+  const uint32_t q_u = smem_u32(Qs), k_u = smem_u32(Ks), v_u = smem_u32(Vs);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int qb = (int)(gridDim.x - 1 - blockIdx.x), bh = blockIdx.y;   // long rows first
   const int b = bh / a.H, h = bh - b * a.H;
-  const int q0 = qb * BQ;
-  const T *qp = (const T *)a.q + b * a.q_sb + h * a.q_sh;
-  const T *kp = (const T *)a.k + b * a.q_sb + h * a.q_sh;
-  const T *vp = (const T *)a.v + b * a.q_sb + h * a.q_sh;
-  load_rows<T, D>(Qs, qp, a.q_st, q0, a.T);
-  float m[4], l[4], o[4][CPT];
+  const int q0 = qb * BQ, row0 = q0 + warp * 16 + lane / 4;            // this thread's rows: row0 and row0 + 8
+  const int64_t off = b * a.q_sb + h * a.q_sh;
+  const T *qp = (const T *)a.q + off, *kp = (const T *)a.k + off, *vp = (const T *)a.v + off;
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  const bool q_big = load_tile<T, D>(Qs, qp, a.q_st, q0, a.T, a.vec_q);
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[D / 8][4];
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    m[i] = -INFINITY;
-    l[i] = 0.f;
+  for (int n = 0; n < D / 8; n++)
 #pragma unroll
-    for (int j = 0; j < CPT; j++) o[i][j] = 0.f;
-  }
+    for (int i = 0; i < 4; i++) o[n][i] = 0.f;
   for (int kb = 0; kb <= qb; kb++) {
     const int k0 = kb * BKV;
     __syncthreads();
-    load_rows_t<T, D>(Kt, kp, a.q_st, k0, a.T);
-    load_rows<T, D>(Vs, vp, a.q_st, k0, a.T);
-    __syncthreads();
-    float s[4][4];
-    tile_abt<D>(s, Qs, Kt, ty, tx);
+    const bool k_big = load_tile<T, D>(Ks, kp, a.q_st, k0, a.T, a.vec_q);
+    load_tile<T, D>(Vs, vp, a.q_st, k0, a.T, a.vec_q);
+    const bool big = __syncthreads_or(q_big || k_big);
+    const int groups = kb == qb ? warp + 1 : 4;   // groups of 16 keys at or before the warp's last row
+    float s[8][4];
+    score_product<T, D, 8>(s, q_u, warp * 16, k_u, 0, 0, groups, lane);
+    if (L::NT > 1 && big) fix_scores<T, D, 8>(s, qp, kp, a.q_st, a.q_st, q0 + warp * 16, k0, a.T);
+    float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int qi = q0 + ty * 4 + i;
-      float mloc = -INFINITY;
+    for (int n = 0; n < 8; n++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int kj = k0 + tx * 4 + j;
-        float x = s[i][j] * a.scale;
-        if (a.cap > 0.f) x = a.cap * tanhf(x / a.cap);
+      for (int i = 0; i < 4; i++) {
+        const int qi = row0 + (i >> 1) * 8, kj = k0 + n * 8 + (lane & 3) * 2 + (i & 1);
+        float x = a.cap > 0.f ? a.cap * tanhf(s[n][i] * a.cap_arg) : s[n][i] * a.scale;
         if (kj > qi || kj >= a.T) x = -INFINITY;
-        s[i][j] = x;
-        mloc = fmaxf(mloc, x);
+        s[n][i] = x;
+        mx[i >> 1] = fmaxf(mx[i >> 1], x);
       }
-      mloc = half_warp_max(mloc);
-      const float mnew = fmaxf(m[i], mloc);
-      const float corr = (mnew == -INFINITY) ? 1.f : expf(m[i] - mnew);
-      float lsum = 0.f;
+    float corr[2];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float p = (mnew == -INFINITY) ? 0.f : expf(s[i][j] - mnew);
-        Ps[(ty * 4 + i) * (64 + PAD) + tx * 4 + j] = p;
-        lsum += p;
-      }
-      lsum = half_warp_sum(lsum);
-      l[i] = l[i] * corr + lsum;
-      m[i] = mnew;
+    for (int r = 0; r < 2; r++) {
+      const float mnew = fmaxf(m[r], quad_max(mx[r]));
+      corr[r] = mnew == -INFINITY ? 1.f : expf(m[r] - mnew);
+      float sum = 0.f;
 #pragma unroll
-      for (int j = 0; j < CPT; j++) o[i][j] *= corr;
+      for (int n = 0; n < 8; n++)
+#pragma unroll
+        for (int i = 2 * r; i < 2 * r + 2; i++) {
+          s[n][i] = mnew == -INFINITY ? 0.f : expf(s[n][i] - mnew);
+          sum += s[n][i];
+        }
+      l[r] = l[r] * corr[r] + quad_sum(sum);
+      m[r] = mnew;
     }
-    __syncthreads();
-    tile_wx<D, false>(o, Ps, Vs, ty, tx);
+    LeftTerms<4> p;
+    p.set(s);
+    output_product<T, D, 4, true>(o, p, v_u, 0, 0, groups, corr[0], corr[1], lane);
   }
   T *op = (T *)a.out_o + b * a.o_sb + h * a.o_sh;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int qi = q0 + ty * 4 + i;
+  for (int r = 0; r < 2; r++) {
+    const int qi = row0 + r * 8;
     if (qi >= a.T) continue;
-    const float inv = 1.f / l[i];
+    const float inv = 1.f / l[r];
 #pragma unroll
-    for (int j = 0; j < CPT; j++) op[(int64_t)qi * a.o_st + tx * CPT + j] = from_f32<T>(o[i][j] * inv);
-    if (tx == 0) a.lse[(int64_t)bh * a.T + qi] = m[i] + logf(l[i]);
+    for (int n = 0; n < D / 8; n++)
+      store_pair(op + (int64_t)qi * a.o_st + n * 8 + (lane & 3) * 2, o[n][2 * r] * inv, o[n][2 * r + 1] * inv, a.vec_o);
+    if ((lane & 3) == 0) a.lse[(int64_t)bh * a.T + qi] = m[r] + logf(l[r]);
   }
 }
 
@@ -195,157 +383,174 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(AttnArgs a, int D, int6
   }
 }
 
-// Recomputes, for the tile (q0, k0): P -> Ps (optional) and dS -> dSs, both [q][key].
-template <int D>
-__device__ __forceinline__ void recompute_p_ds(const AttnArgs &a, const float *Qs, const float *Kt, const float *dOs,
-                                               const float *Vt, const float *lse_s, const float *delta_s, float *Ps,
-                                               float *dSs, int q0, int k0, int ty, int tx) {
-  float s[4][4], dp[4][4];
-  tile_abt<D>(s, Qs, Kt, ty, tx);
-  tile_abt<D>(dp, dOs, Vt, ty, tx);
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int qi = q0 + ty * 4 + i;
-    const float lse = lse_s[ty * 4 + i], dl = delta_s[ty * 4 + i];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int kj = k0 + tx * 4 + j;
-      float x = s[i][j] * a.scale, dcap = 1.f;
-      if (a.cap > 0.f) {
-        const float th = tanhf(x / a.cap);
-        x = a.cap * th;
-        dcap = 1.f - th * th;
-      }
-      const bool dead = kj > qi || kj >= a.T || qi >= a.T;
-      const float p = dead ? 0.f : expf(x - lse);
-      const float ds = p * (dp[i][j] - dl) * dcap * a.scale;
-      if (Ps) Ps[(ty * 4 + i) * (64 + PAD) + tx * 4 + j] = p;
-      dSs[(ty * 4 + i) * (64 + PAD) + tx * 4 + j] = ds;
-    }
+// From raw score s and dP of (query qi, key kj): P and dS.
+__device__ __forceinline__ void p_and_ds(const AttnArgs &a, float s, float dp, float lse, float delta, int qi, int kj,
+                                         float &p, float &ds) {
+  float x = s * a.scale, dcap = 1.f;
+  if (a.cap > 0.f) {
+    const float th = tanhf(s * a.cap_arg);
+    x = a.cap * th;
+    dcap = 1.f - th * th;
   }
+  p = kj > qi || qi >= a.T ? 0.f : expf(x - lse);   // kj <= qi < T
+  ds = p * (dp - delta) * dcap * a.scale;
 }
 
+// dK, dV of 64 keys: the warp's rows are keys, so the products run on S^T and dP^T, 32 queries at a time.
 template <typename T, int D>
-__global__ void __launch_bounds__(256) attn_bwd_dkv_kernel(AttnArgs a) {
-  extern __shared__ __align__(16) float sm[];
-  constexpr int CPT = D / 16;
-  float *Kt = sm;                           // [D][64+PAD]
-  float *Vt = Kt + D * (64 + PAD);          // [D][64+PAD]
-  float *Qs = Vt + D * (64 + PAD);          // [64][D+PAD]
-  float *dOs = Qs + 64 * (D + PAD);         // [64][D+PAD]
-  float *Ps = dOs + 64 * (D + PAD);         // [64][64+PAD]
-  float *dSs = Ps + 64 * (64 + PAD);        // [64][64+PAD]
-  float *lse_s = dSs + 64 * (64 + PAD);     // [64]
-  float *delta_s = lse_s + 64;              // [64]
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int kb = blockIdx.x, bh = blockIdx.y;
+__global__ void __launch_bounds__(ATTN_THREADS) attn_bwd_dkv_kernel(const AttnArgs a) {
+  using L = AttnTile<T, D>;
+  extern __shared__ __align__(16) uint8_t at_sm[];
+  uint8_t *Ks = at_sm, *Vs = Ks + L::BYTES, *Qs = Vs + L::BYTES, *dOs = Qs + L::BYTES;
+  float *lse_s = reinterpret_cast<float *>(dOs + L::BYTES), *delta_s = lse_s + 64;
+  const uint32_t k_u = smem_u32(Ks), v_u = smem_u32(Vs), q_u = smem_u32(Qs), do_u = smem_u32(dOs);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kb = blockIdx.x, bh = blockIdx.y;   // kb 0 meets the most queries and comes first
   const int b = bh / a.H, h = bh - b * a.H;
-  const int k0 = kb * BKV;
+  const int k0 = kb * BKV, row0 = k0 + warp * 16 + lane / 4;
   const int64_t qoff = b * a.q_sb + h * a.q_sh, ooff = b * a.o_sb + h * a.o_sh;
-  load_rows_t<T, D>(Kt, (const T *)a.k + qoff, a.q_st, k0, a.T);
-  load_rows_t<T, D>(Vt, (const T *)a.v + qoff, a.q_st, k0, a.T);
-  float dk[4][CPT], dv[4][CPT];
+  const T *qp = (const T *)a.q + qoff, *kp = (const T *)a.k + qoff, *vp = (const T *)a.v + qoff, *dop = (const T *)a.d_o + ooff;
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  bool kv_big = load_tile<T, D>(Ks, kp, a.q_st, k0, a.T, a.vec_q);
+  kv_big |= load_tile<T, D>(Vs, vp, a.q_st, k0, a.T, a.vec_q);
+  float dk[D / 8][4], dv[D / 8][4];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int n = 0; n < D / 8; n++)
 #pragma unroll
-    for (int j = 0; j < CPT; j++) dk[i][j] = dv[i][j] = 0.f;
+    for (int i = 0; i < 4; i++) dk[n][i] = dv[n][i] = 0.f;
   const int n_qb = (a.T + BQ - 1) / BQ;
   for (int qb = kb; qb < n_qb; qb++) {
     const int q0 = qb * BQ;
     __syncthreads();
-    load_rows<T, D>(Qs, (const T *)a.q + qoff, a.q_st, q0, a.T);
-    load_rows<T, D>(dOs, (const T *)a.d_o + ooff, a.o_st, q0, a.T);
+    bool q_big = load_tile<T, D>(Qs, qp, a.q_st, q0, a.T, a.vec_q);
+    q_big |= load_tile<T, D>(dOs, dop, a.o_st, q0, a.T, a.vec_o);
     if (threadIdx.x < 64) {
       const int t = q0 + threadIdx.x;
       lse_s[threadIdx.x] = t < a.T ? a.lse_in[(int64_t)bh * a.T + t] : 0.f;
       delta_s[threadIdx.x] = t < a.T ? a.delta[(int64_t)bh * a.T + t] : 0.f;
     }
-    __syncthreads();
-    recompute_p_ds<D>(a, Qs, Kt, dOs, Vt, lse_s, delta_s, Ps, dSs, q0, k0, ty, tx);
-    __syncthreads();
-    tile_wx<D, true>(dv, Ps, dOs, ty, tx);   // dV[key] += sum_q P[q][key] dO[q]
-    tile_wx<D, true>(dk, dSs, Qs, ty, tx);   // dK[key] += sum_q dS[q][key] Q[q]
+    const bool big = __syncthreads_or(kv_big || q_big);
+#pragma unroll 1
+    for (int c = 0; c < 64; c += 32) {
+      const int from = qb == kb ? max(warp - c / 16, 0) : 0;   // groups of 16 queries before the warp's first key: nothing
+      if (from >= 2) continue;
+      float s[4][4], dp[4][4];
+      score_product<T, D, 4>(s, k_u, warp * 16, q_u, c, from, 2, lane);
+      score_product<T, D, 4>(dp, v_u, warp * 16, do_u, c, from, 2, lane);
+      if (L::NT > 1 && big) {
+        fix_scores<T, D, 4>(s, kp, qp, a.q_st, a.q_st, k0 + warp * 16, q0 + c, a.T);
+        fix_scores<T, D, 4>(dp, vp, dop, a.q_st, a.o_st, k0 + warp * 16, q0 + c, a.T);
+      }
+#pragma unroll
+      for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int qc = c + n * 8 + (lane & 3) * 2 + (i & 1);
+          p_and_ds(a, s[n][i], dp[n][i], lse_s[qc], delta_s[qc], q0 + qc, row0 + (i >> 1) * 8, s[n][i], dp[n][i]);
+        }
+      LeftTerms<2> w;
+      w.set(s);
+      output_product<T, D, 2, false>(dv, w, do_u, c, from, 2, 1.f, 1.f, lane);   // dV[key] += sum_q P[q][key] dO[q]
+      w.set(dp);
+      output_product<T, D, 2, false>(dk, w, q_u, c, from, 2, 1.f, 1.f, lane);    // dK[key] += sum_q dS[q][key] Q[q]
+    }
   }
   T *dkp = (T *)a.dk + qoff, *dvp = (T *)a.dv + qoff;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int kj = k0 + ty * 4 + i;
+  for (int r = 0; r < 2; r++) {
+    const int kj = row0 + r * 8;
     if (kj >= a.T) continue;
 #pragma unroll
-    for (int j = 0; j < CPT; j++) {
-      dkp[(int64_t)kj * a.q_st + tx * CPT + j] = from_f32<T>(dk[i][j]);
-      dvp[(int64_t)kj * a.q_st + tx * CPT + j] = from_f32<T>(dv[i][j]);
+    for (int n = 0; n < D / 8; n++) {
+      const int64_t at = (int64_t)kj * a.q_st + n * 8 + (lane & 3) * 2;
+      store_pair(dkp + at, dk[n][2 * r], dk[n][2 * r + 1], a.vec_q);
+      store_pair(dvp + at, dv[n][2 * r], dv[n][2 * r + 1], a.vec_q);
     }
   }
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(256) attn_bwd_dq_kernel(AttnArgs a) {
-  extern __shared__ __align__(16) float sm[];
-  constexpr int CPT = D / 16;
-  float *Kt = sm;                           // [D][64+PAD]
-  float *Vt = Kt + D * (64 + PAD);          // [D][64+PAD]
-  float *Qs = Vt + D * (64 + PAD);          // [64][D+PAD]
-  float *dOs = Qs + 64 * (D + PAD);         // [64][D+PAD]
-  float *Ks = dOs + 64 * (D + PAD);         // [64][D+PAD]
-  float *dSs = Ks + 64 * (D + PAD);         // [64][64+PAD]
-  float *lse_s = dSs + 64 * (64 + PAD);
-  float *delta_s = lse_s + 64;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int qb = blockIdx.x, bh = blockIdx.y;
+__global__ void __launch_bounds__(ATTN_THREADS) attn_bwd_dq_kernel(const AttnArgs a) {
+  using L = AttnTile<T, D>;
+  extern __shared__ __align__(16) uint8_t at_sm[];
+  uint8_t *Ks = at_sm, *Vs = Ks + L::BYTES, *Qs = Vs + L::BYTES, *dOs = Qs + L::BYTES;
+  const uint32_t k_u = smem_u32(Ks), v_u = smem_u32(Vs), q_u = smem_u32(Qs), do_u = smem_u32(dOs);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int qb = (int)(gridDim.x - 1 - blockIdx.x), bh = blockIdx.y;
   const int b = bh / a.H, h = bh - b * a.H;
-  const int q0 = qb * BQ;
+  const int q0 = qb * BQ, row0 = q0 + warp * 16 + lane / 4;
   const int64_t qoff = b * a.q_sb + h * a.q_sh, ooff = b * a.o_sb + h * a.o_sh;
-  load_rows<T, D>(Qs, (const T *)a.q + qoff, a.q_st, q0, a.T);
-  load_rows<T, D>(dOs, (const T *)a.d_o + ooff, a.o_st, q0, a.T);
-  if (threadIdx.x < 64) {
-    const int t = q0 + threadIdx.x;
-    lse_s[threadIdx.x] = t < a.T ? a.lse_in[(int64_t)bh * a.T + t] : 0.f;
-    delta_s[threadIdx.x] = t < a.T ? a.delta[(int64_t)bh * a.T + t] : 0.f;
+  const T *qp = (const T *)a.q + qoff, *kp = (const T *)a.k + qoff, *vp = (const T *)a.v + qoff, *dop = (const T *)a.d_o + ooff;
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  bool q_big = load_tile<T, D>(Qs, qp, a.q_st, q0, a.T, a.vec_q);
+  q_big |= load_tile<T, D>(dOs, dop, a.o_st, q0, a.T, a.vec_o);
+  float lse[2], delta[2];
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const int t = row0 + r * 8;
+    lse[r] = t < a.T ? a.lse_in[(int64_t)bh * a.T + t] : 0.f;
+    delta[r] = t < a.T ? a.delta[(int64_t)bh * a.T + t] : 0.f;
   }
-  float dq[4][CPT];
+  float dq[D / 8][4];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int n = 0; n < D / 8; n++)
 #pragma unroll
-    for (int j = 0; j < CPT; j++) dq[i][j] = 0.f;
+    for (int i = 0; i < 4; i++) dq[n][i] = 0.f;
   for (int kb = 0; kb <= qb; kb++) {
     const int k0 = kb * BKV;
     __syncthreads();
-    load_rows_t<T, D>(Kt, (const T *)a.k + qoff, a.q_st, k0, a.T);
-    load_rows_t<T, D>(Vt, (const T *)a.v + qoff, a.q_st, k0, a.T);
-    load_rows<T, D>(Ks, (const T *)a.k + qoff, a.q_st, k0, a.T);
-    __syncthreads();
-    recompute_p_ds<D>(a, Qs, Kt, dOs, Vt, lse_s, delta_s, nullptr, dSs, q0, k0, ty, tx);
-    __syncthreads();
-    tile_wx<D, false>(dq, dSs, Ks, ty, tx);  // dQ[q] += sum_key dS[q][key] K[key]
+    bool kv_big = load_tile<T, D>(Ks, kp, a.q_st, k0, a.T, a.vec_q);
+    kv_big |= load_tile<T, D>(Vs, vp, a.q_st, k0, a.T, a.vec_q);
+    const bool big = __syncthreads_or(q_big || kv_big);
+#pragma unroll 1
+    for (int c = 0; c < 64; c += 32) {
+      const int to = kb == qb ? min(warp + 1 - c / 16, 2) : 2;   // groups of 16 keys at or before the warp's last row
+      if (to <= 0) continue;
+      float s[4][4], dp[4][4];
+      score_product<T, D, 4>(s, q_u, warp * 16, k_u, c, 0, to, lane);
+      score_product<T, D, 4>(dp, do_u, warp * 16, v_u, c, 0, to, lane);
+      if (L::NT > 1 && big) {
+        fix_scores<T, D, 4>(s, qp, kp, a.q_st, a.q_st, q0 + warp * 16, k0 + c, a.T);
+        fix_scores<T, D, 4>(dp, dop, vp, a.o_st, a.q_st, q0 + warp * 16, k0 + c, a.T);
+      }
+#pragma unroll
+      for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          float p;
+          p_and_ds(a, s[n][i], dp[n][i], lse[i >> 1], delta[i >> 1], row0 + (i >> 1) * 8,
+                   k0 + c + n * 8 + (lane & 3) * 2 + (i & 1), p, dp[n][i]);
+        }
+      LeftTerms<2> w;
+      w.set(dp);
+      output_product<T, D, 2, false>(dq, w, k_u, c, 0, to, 1.f, 1.f, lane);   // dQ[q] += sum_key dS[q][key] K[key]
+    }
   }
   T *dqp = (T *)a.dq + qoff;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int qi = q0 + ty * 4 + i;
+  for (int r = 0; r < 2; r++) {
+    const int qi = row0 + r * 8;
     if (qi >= a.T) continue;
 #pragma unroll
-    for (int j = 0; j < CPT; j++) dqp[(int64_t)qi * a.q_st + tx * CPT + j] = from_f32<T>(dq[i][j]);
+    for (int n = 0; n < D / 8; n++)
+      store_pair(dqp + (int64_t)qi * a.q_st + n * 8 + (lane & 3) * 2, dq[n][2 * r], dq[n][2 * r + 1], a.vec_q);
   }
 }
 
-template <int D> constexpr size_t fwd_smem() { return sizeof(float) * (2 * 64 * (D + PAD) + D * (64 + PAD) + 64 * (64 + PAD)); }
-template <int D> constexpr size_t dkv_smem() {
-  return sizeof(float) * (2 * D * (64 + PAD) + 2 * 64 * (D + PAD) + 2 * 64 * (64 + PAD) + 128);
-}
-template <int D> constexpr size_t dq_smem() {
-  return sizeof(float) * (2 * D * (64 + PAD) + 3 * 64 * (D + PAD) + 64 * (64 + PAD) + 128);
-}
+template <typename T, int D> constexpr size_t fwd_smem() { return 3 * AttnTile<T, D>::BYTES; }
+template <typename T, int D> constexpr size_t bwd_smem() { return 4 * AttnTile<T, D>::BYTES + 128 * sizeof(float); }
 
 template <typename T, int D>
 static int fwd_launch(const AttnArgs &a, int64_t batch) {
   static int attr = -1;
   if (attr != g_init_epoch) {
-    ALPHA_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem<D>()));
+    ALPHA_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem<T, D>()));
     attr = g_init_epoch;
   }
   dim3 grid((unsigned)((a.T + BQ - 1) / BQ), (unsigned)(batch * a.H));
-  attn_fwd_kernel<T, D><<<grid, 256, fwd_smem<D>(), g_stream>>>(a);
+  ALPHA_CUDA(launch_overlapped(OVL_ATTN_FWD, attn_fwd_kernel<T, D>, grid, dim3(ATTN_THREADS), fwd_smem<T, D>(), a));
   ALPHA_LAUNCHED();
   return 0;
 }
@@ -354,17 +559,17 @@ template <typename T, int D>
 static int bwd_launch(const AttnArgs &a, int64_t batch) {
   static int attr = -1;
   if (attr != g_init_epoch) {
-    ALPHA_CUDA(cudaFuncSetAttribute(attn_bwd_dkv_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dkv_smem<D>()));
-    ALPHA_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq_smem<D>()));
+    ALPHA_CUDA(cudaFuncSetAttribute(attn_bwd_dkv_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem<T, D>()));
+    ALPHA_CUDA(cudaFuncSetAttribute(attn_bwd_dq_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem<T, D>()));
     attr = g_init_epoch;
   }
   const int64_t rows = batch * a.H * a.T;
   attn_delta_kernel<T><<<grid_for(rows, 8, 8), 256, 0, g_stream>>>(a, D, rows);
   g_launches++;
   dim3 grid((unsigned)((a.T + BQ - 1) / BQ), (unsigned)(batch * a.H));
-  attn_bwd_dkv_kernel<T, D><<<grid, 256, dkv_smem<D>(), g_stream>>>(a);
+  ALPHA_CUDA(launch_overlapped(OVL_ATTN_BWD, attn_bwd_dkv_kernel<T, D>, grid, dim3(ATTN_THREADS), bwd_smem<T, D>(), a));
   g_launches++;
-  attn_bwd_dq_kernel<T, D><<<grid, 256, dq_smem<D>(), g_stream>>>(a);
+  ALPHA_CUDA(launch_overlapped(OVL_ATTN_BWD, attn_bwd_dq_kernel<T, D>, grid, dim3(ATTN_THREADS), bwd_smem<T, D>(), a));
   ALPHA_LAUNCHED();
   return 0;
 }
@@ -378,14 +583,25 @@ static int check_params(const alpha_attn_params_t *p, const char *who) {
   return 0;
 }
 
+// Strides and scale factors, and whether four consecutive elements can move at once.
+static void set_geometry(AttnArgs &a, const alpha_attn_params_t *p) {
+  a.q_sb = p->q_sb; a.q_sh = p->q_sh; a.q_st = p->q_st; a.o_sb = p->o_sb; a.o_sh = p->o_sh; a.o_st = p->o_st;
+  a.H = (int)p->heads; a.T = (int)p->T; a.scale = p->scale; a.cap = p->soft_cap;
+  a.cap_arg = p->soft_cap > 0.f ? (float)((double)p->scale / (double)p->soft_cap) : 0.f;
+  const uintptr_t mask = 4 * dtype_size(p->dtype) - 1;
+  const uintptr_t q_all = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.dq | (uintptr_t)a.dk | (uintptr_t)a.dv;
+  const uintptr_t o_all = (uintptr_t)a.d_o | (uintptr_t)a.out_o;
+  a.vec_q = (q_all & mask) == 0 && p->q_st % 4 == 0 && (p->heads == 1 || p->q_sh % 4 == 0) && (p->batch == 1 || p->q_sb % 4 == 0);
+  a.vec_o = (o_all & mask) == 0 && p->o_st % 4 == 0 && (p->heads == 1 || p->o_sh % 4 == 0) && (p->batch == 1 || p->o_sb % 4 == 0);
+}
+
 int attn_f32_fwd(alpha_buf q, alpha_buf k, alpha_buf v, alpha_buf o, alpha_buf lse, const alpha_attn_params_t *p) {
   if (check_params(p, "alpha_flash_attn_fwd")) return 1;
   if (p->batch * p->heads * p->T == 0) return 0;
   ProfScope prof(PROF_ATTN_FWD, 4.0 * p->batch * p->heads * (double)p->T * p->T * p->D);
   AttnArgs a{};
   a.q = ptr<void>(q); a.k = ptr<void>(k); a.v = ptr<void>(v); a.out_o = ptr<void>(o); a.lse = ptr<float>(lse);
-  a.q_sb = p->q_sb; a.q_sh = p->q_sh; a.q_st = p->q_st; a.o_sb = p->o_sb; a.o_sh = p->o_sh; a.o_st = p->o_st;
-  a.H = (int)p->heads; a.T = (int)p->T; a.scale = p->scale; a.cap = p->soft_cap;
+  set_geometry(a, p);
 #define FWD_CASE(DD)                                                                      \
   case DD:                                                                                \
     return p->dtype == ALPHA_F32 ? fwd_launch<float, DD>(a, p->batch) : fwd_launch<__nv_bfloat16, DD>(a, p->batch);
@@ -402,8 +618,7 @@ int attn_f32_bwd(alpha_buf q, alpha_buf k, alpha_buf v, alpha_buf o, alpha_buf d
   AttnArgs a{};
   a.q = ptr<void>(q); a.k = ptr<void>(k); a.v = ptr<void>(v); a.o = ptr<void>(o); a.d_o = ptr<void>(d_o);
   a.lse_in = ptr<float>(lse); a.dq = ptr<void>(dq); a.dk = ptr<void>(dk); a.dv = ptr<void>(dv);
-  a.q_sb = p->q_sb; a.q_sh = p->q_sh; a.q_st = p->q_st; a.o_sb = p->o_sb; a.o_sh = p->o_sh; a.o_st = p->o_st;
-  a.H = (int)p->heads; a.T = (int)p->T; a.scale = p->scale; a.cap = p->soft_cap;
+  set_geometry(a, p);
   void *delta = nullptr;
   if (pool_alloc((size_t)p->batch * p->heads * p->T * sizeof(float), &delta)) return 1;
   a.delta = (float *)delta;

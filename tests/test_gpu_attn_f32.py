@@ -1,0 +1,118 @@
+"""fp32-accurate attention (three bf16 terms per number on the tensor cores) against 64 bits.
+
+Bounds, with u = 2^-24.  A product of two fp32 vectors of length n here is off by at most c(n)*u times the
+product of their magnitudes, c(n) = 2*6*n/16 + 8 (six truncating adds per 16 terms, 2u each, and the
+splits) inside a tile and one rounding per 32 keys between tiles.  A score error d moves a probability by
+the factor e^d, so P is off by (2*max|d| + 16u) relatively (tanh and exp are good to a few u), and the
+outputs by that plus the product's own error.  bf16 results are rounded once more: 2^-8 of the value.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -24
+
+
+@pytest.fixture(scope="module")
+def B():
+    from alpha2_b200.backend import CudaBackend
+    b = CudaBackend(0)
+    yield b
+    b.checkAsyncError()
+
+
+def reference(q, k, v, do, scale, cap):
+    """Values and error bounds of one head in 64 bits: o, lse, dq, dk, dv."""
+    T, D = q.shape
+    s = q @ k.T * scale
+    th = np.tanh(s / cap) if cap else np.zeros_like(s)
+    x = cap * th if cap else s
+    dcap = 1 - th ** 2
+    dead = np.triu(np.ones((T, T), bool), 1)
+    x = np.where(dead, -np.inf, x)
+    lse = np.log(np.exp(x - x.max(1, keepdims=True)).sum(1)) + x.max(1)
+    p = np.exp(x - lse[:, None])
+    o = p @ v
+    delta = (o * do).sum(1)
+    dp = do @ v.T
+    ds = p * (dp - delta[:, None]) * dcap * scale
+    cD, cT = (0.75 * max(D, 16) + 8) * U, (0.75 * 64 + 8 + T / 32) * U
+    d = (np.where(dead, 0, cD * (np.abs(q) @ np.abs(k).T) * scale + 4 * U * np.abs(s))).max()
+    pe = 2 * d + 16 * U + T / 16 * U           # relative error of P: scores, exp, the row sum
+    oe = (pe + cT) * (p @ np.abs(v))
+    dse = p * scale * (np.abs(dp - delta[:, None]) * (pe + 4 * d + 16 * U)
+                       + (cD + 4 * U) * (np.abs(do) @ np.abs(v).T) + ((np.abs(o) + 1) * np.abs(do)).sum(1)[:, None] * (cD + pe + cT))
+    return ((o, oe), (lse, d + (16 + T / 16) * U * (1 + np.abs(lse))), (ds @ k, dse @ np.abs(k) + cT * (np.abs(ds) @ np.abs(k))),
+            (ds.T @ q, dse.T @ np.abs(q) + cT * (np.abs(ds).T @ np.abs(q))),
+            (p.T @ do, (pe + cT) * (p.T @ np.abs(do))))
+
+
+def data(BH, T, D, dtype, seed):
+    from alpha2_b200.backend import bf16_to_f32, f32_to_bf16_bits
+    g = np.random.default_rng(seed)
+    out = [g.standard_normal((BH, T, D)).astype(np.float32) for _ in range(4)]
+    return [bf16_to_f32(f32_to_bf16_bits(t)).reshape(t.shape) for t in out] if dtype == "bf16" else out
+
+
+# one short of, at and one past the 16-row groups and 64-row tiles; every head size
+@pytest.mark.parametrize("D", [16, 32, 64, 128])
+@pytest.mark.parametrize("T", [1, 2, 15, 17, 32, 63, 64, 65, 129, 300])
+@pytest.mark.parametrize("dtype,cap", [("f32", 30.0), ("f32", 0.0), ("bf16", 2.0)])
+def test_against_64_bits(B, D, T, dtype, cap):
+    if dtype == "bf16" and D == 64:
+        pytest.skip("bf16 with head dimension 64 has kernels of its own")
+    q, k, v, do = data(2, T, D, dtype, T * D)
+    scale = D ** -0.5
+    Q, K, V, dO = (B.upload(t, dtype) for t in (q, k, v, do))
+    res = B.flashAttention(Q, K, V, T, scale, cap)
+    o = np.array(res["output"].data, np.float64)
+    g = B.flashAttentionBackward(Q, K, V, res["output"], dO, res["lse"], T, scale, cap)
+    got = [o, np.array(res["lse"].data, np.float64)] + [np.array(g[n].data, np.float64) for n in ("dQ", "dK", "dV")]
+    extra = 2.0 ** -8 if dtype == "bf16" else 0.0
+    for h in range(2):
+        ref = reference(*(t[h].astype(np.float64) for t in (q, k, v, do)), scale, cap)
+        # bf16: the rounded output enters D_i: dS is off by up to 2^-9 (|o| . |dO|) p scale
+        dd = 2.0 ** -9 * (np.abs(ref[0][0]) * np.abs(do[h])).sum(1).max() * scale if dtype == "bf16" else 0.0
+        slack = {"dQ": dd * np.abs(k[h]).max(), "dK": dd * np.abs(q[h]).max() * T}
+        for name, x, (want, err) in zip(("o", "lse", "dQ", "dK", "dV"), got, ref):
+            e = err + (extra * np.abs(want) + slack.get(name, 0.0) if name != "lse" else 0.0)
+            assert np.all(np.abs(x[h] - want) <= e + 1e-30), (name, float((np.abs(x[h] - want) / (e + 1e-30)).max()))
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("pad", [1, 2, 4])      # row strides that lose and keep 8- and 16-byte access
+def test_row_strides(B, dtype, pad):
+    """q, k, v and their gradients with rows `pad` elements longer than their data: the same bits as dense."""
+    import ctypes as C
+    from alpha2_b200 import _lib as L
+    from alpha2_b200._lib import check
+    BH, T, D = 3, 70, 32
+    q, k, v, do = data(BH, T, D, dtype, 5)
+    dense = [B.upload(t, dtype) for t in (q, k, v, do)]
+    r = B.flashAttention(*dense[:3], T, 0.2, 30.0)
+    g = B.flashAttentionBackward(*dense[:3], r["output"], dense[3], r["lse"], T, 0.2, 30.0)
+    ld = D + pad
+    padded = [B.upload(np.concatenate([t, np.full((BH, T, pad), 9, np.float32)], 2), dtype) for t in (q, k, v, do)]
+    p = L.AttnParams(batch=BH, heads=1, T=T, D=D, q_sb=T * ld, q_sh=0, q_st=ld, o_sb=T * ld, o_sh=0, o_st=ld, scale=0.2,
+                     soft_cap=30.0, dtype=L.DTYPE_CODE[dtype])
+    out, dq, dk, dv = (B.zeros((BH, T, ld), dtype) for _ in range(4))
+    lse = B.zeros((BH, T), "f32")
+    check(B.lib.alpha_flash_attn_fwd(*(t.ptr for t in padded[:3]), out.ptr, lse.ptr, C.byref(p)))
+    check(B.lib.alpha_flash_attn_bwd(*(t.ptr for t in padded[:3]), out.ptr, padded[3].ptr, lse.ptr, dq.ptr, dk.ptr, dv.ptr,
+                                     C.byref(p)))
+    for got, want in ((out, r["output"]), (dq, g["dQ"]), (dk, g["dK"]), (dv, g["dV"])):
+        x = np.array(got.data)
+        assert np.array_equal(x[:, :, :D], np.array(want.data)) and not x[:, :, D:].any()
+
+
+def test_infinite_scores_meet_the_cap(B):
+    """An infinity in q or k makes its scores +-inf, which the soft cap maps to +-cap; other rows are untouched."""
+    T, D = 96, 32
+    q, k, v, do = data(1, T, D, "f32", 8)
+    k[:, :, 4] = np.abs(k[:, :, 4]) + 0.1
+    clean = np.array(B.flashAttention(*(B.upload(t, "f32") for t in (q, k, v)), T, 0.2, 30.0)["output"].data)
+    q[0, 70, 4] = np.inf
+    got = np.array(B.flashAttention(*(B.upload(t, "f32") for t in (q, k, v)), T, 0.2, 30.0)["output"].data)
+    assert np.allclose(got[0, 70], v[0, :71].mean(0), rtol=1e-5, atol=1e-6)     # every score at the cap: the mean
+    assert np.array_equal(np.delete(got, 70, 1), np.delete(clean, 70, 1))
