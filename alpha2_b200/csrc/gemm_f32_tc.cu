@@ -25,7 +25,7 @@
 // warps flag such a tile, and its elements that came out non-finite are recomputed with an fmaf
 // chain in K order.  NaN operands need nothing: the result is NaN either way.
 //
-// Measured on a B200: 8192 x 4096 x 384 in 248 us (104 TFLOP/s), 16384 x 768 x 256 in 82 us (79); an
+// Measured on a B200: 8192 x 4096 x 384 in 199 us (130 TFLOP/s), 16384 x 768 x 256 in 64 us (100); an
 // FMA-pipe kernel with 4 x 4 outputs per thread ran such products at 9 to 15 TFLOP/s.  Bound by the operand
 // warps (splitting and the loads it waits for), not by the tensor core.
 #include <string.h>
@@ -67,11 +67,17 @@ struct F3Layout {
 };
 
 // x = h + m + l for a pair; each result holds the pair's two bf16 terms
+__device__ __forceinline__ uint64_t minus_terms(uint64_t x, uint32_t t) {   // exact: t is x rounded
+  return f2_fma(bf16x2_to_f2(t), f2_pack(-1.f, -1.f), x);
+}
 __device__ __forceinline__ void split3(float x0, float x1, uint32_t &h, uint32_t &m, uint32_t &l) {
+  float r0, r1;
   h = bf16x2_pack(x0, x1);
-  const float r0 = x0 - __uint_as_float(h << 16), r1 = x1 - __uint_as_float(h & 0xFFFF0000u);
+  const uint64_t r = minus_terms(f2_pack(x0, x1), h);
+  f2_unpack(r, r0, r1);
   m = bf16x2_pack(r0, r1);
-  l = bf16x2_pack(r0 - __uint_as_float(m << 16), r1 - __uint_as_float(m & 0xFFFF0000u));
+  f2_unpack(minus_terms(r, m), r0, r1);
+  l = bf16x2_pack(r0, r1);
 }
 
 // One operand tile of ROWS (M or N) x 64 (K) on its way from global to shared memory, shared by
@@ -90,12 +96,19 @@ struct F3Operand {
     return MN ? i * (1024 / ROWS) + tid / (ROWS / 4) : (tid % 16) * 4;
   }
   __device__ __forceinline__ void load(const float *p, int64_t ld, int r0, int rows, int k0, int K, int vec, int tid) {
+    p += MN ? (int64_t)(k0 + k_of(tid, 0)) * ld + (r0 + row_of(tid, 0)) : (int64_t)(r0 + row_of(tid, 0)) * ld + (k0 + k_of(tid, 0));
+    const int64_t step = (MN ? 1024 / ROWS : 16) * ld;
+    if (vec && r0 + ROWS <= rows && k0 + F3_BK <= K) {   // the whole tile lies inside
+#pragma unroll
+      for (int i = 0; i < PASSES; i++) r[i] = *reinterpret_cast<const float4 *>(p + i * step);
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < PASSES; i++) {
       const int row = r0 + row_of(tid, i), k = k0 + k_of(tid, i);
       const int c = MN ? row : k, c_end = MN ? rows : K;        // contiguous coordinate and its limit
       const bool in = MN ? k < K : row < rows;
-      const float *src = p + (MN ? (int64_t)k * ld + row : (int64_t)row * ld + k);
+      const float *src = p + i * step;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (vec && in && c + 4 <= c_end) {
         v = *reinterpret_cast<const float4 *>(src);
@@ -110,24 +123,25 @@ struct F3Operand {
   }
   // Returns whether the thread's elements hold an infinity or a value from 2^127 on.
   __device__ __forceinline__ bool store(uint8_t *planes, int tid) const {
-    bool big = false;
+    // K-major: rows of 64 k (128 bytes); MN-major: atoms of 64 rows, per atom one 128-byte line per k.  The
+    // 16-byte chunks of a line are swizzled by the line's number modulo 8, which is the same in every pass.
+    const int row = row_of(tid, 0), k = k_of(tid, 0);
+    const uint32_t line = MN ? (uint32_t)((row / 64) * 8192 + k * 128) : (uint32_t)(row * 128);
+    const int at = MN ? row % 64 : k, sw = (MN ? k : row) & 7;
+    planes += line + (uint32_t)(((at >> 3) ^ sw) << 4) + (uint32_t)(at & 7) * 2;
+    constexpr int PASS = (MN ? 1024 / ROWS : 16) * 128;   // bytes between two passes
+    float top = 0.f;
 #pragma unroll
     for (int i = 0; i < PASSES; i++) {
-      const int row = row_of(tid, i), k = k_of(tid, i);
-      // K-major: rows of 64 k (128 bytes); MN-major: atoms of 64 rows, per atom one 128-byte line per k
-      const uint32_t line = MN ? (uint32_t)((row / 64) * 8192 + k * 128) : (uint32_t)(row * 128);
-      const int at = MN ? row % 64 : k, sw = (MN ? k : row) & 7;
-      const uint32_t off = line + (uint32_t)(((at >> 3) ^ sw) << 4) + (uint32_t)(at & 7) * 2;
       uint2 h, m, l;
       split3(r[i].x, r[i].y, h.x, m.x, l.x);
       split3(r[i].z, r[i].w, h.y, m.y, l.y);
-      *reinterpret_cast<uint2 *>(planes + off) = h;
-      *reinterpret_cast<uint2 *>(planes + PLANE + off) = m;
-      *reinterpret_cast<uint2 *>(planes + 2 * PLANE + off) = l;
-      const float big4 = fmaxf(fmaxf(fabsf(r[i].x), fabsf(r[i].y)), fmaxf(fabsf(r[i].z), fabsf(r[i].w)));
-      big |= big4 >= 1.7014118346046923e38f;   // 2^127; a NaN beside it does not hide it (fmaxf drops NaN)
+      *reinterpret_cast<uint2 *>(planes + i * PASS) = h;
+      *reinterpret_cast<uint2 *>(planes + PLANE + i * PASS) = m;
+      *reinterpret_cast<uint2 *>(planes + 2 * PLANE + i * PASS) = l;
+      top = fmax3(top, fmaxf(fabsf(r[i].x), fabsf(r[i].y)), fmaxf(fabsf(r[i].z), fabsf(r[i].w)));
     }
-    return big;
+    return top >= 1.7014118346046923e38f;   // 2^127; a NaN beside it does not hide it (max drops NaN)
   }
 };
 
@@ -314,6 +328,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
       const bool big = big_tag[it % F3_FLAGS] == it + 1;
       float *C = g.C + split * g.split_c + z * g.batch_c;
       const float *aux_in = g.aux_in;
+      const bool plain = g.epilogue == ALPHA_EPI_NONE && !g.accumulate;
       const bool aux_read = g.epilogue == ALPHA_EPI_ADD || g.epilogue == ALPHA_EPI_GELU_BWD;
 #pragma unroll
       for (int c = 0; c < NC; c += 32) {
@@ -329,10 +344,20 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
         __syncwarp();
         // and out again, eight lanes to a row: 128-byte segments
         const int q = lane & 7, n = n_base + c + q * 4;
+        const int rows = min(32, g.M - m_base);
+        float *dst = C + (int64_t)(m_base + (lane >> 3)) * g.ldc + n;
+        int64_t aux_at = (int64_t)(m_base + (lane >> 3)) * g.ld_aux + n;
+        if (g.vec_c && n + 4 <= g.N && !big && plain) {
+#pragma unroll 4
+          for (int rr = lane >> 3; rr < rows; rr += 4, dst += 4 * g.ldc)
+            *reinterpret_cast<float4 *>(dst) = *reinterpret_cast<const float4 *>(stg + rr * 32 + ((q ^ (rr & 7)) << 2));
+          __syncwarp();
+          continue;
+        }
 #pragma unroll 1
-        for (int rr = lane >> 3; rr < 32; rr += 4) {
+        for (int rr = lane >> 3; rr < rows; rr += 4, dst += 4 * g.ldc, aux_at += 4 * g.ld_aux) {
+          if (n >= g.N) continue;
           const int64_t m = m_base + rr;
-          if (m >= g.M || n >= g.N) continue;
           const float4 s4 = *reinterpret_cast<const float4 *>(stg + rr * 32 + ((q ^ (rr & 7)) << 2));
           float v[4] = {s4.x, s4.y, s4.z, s4.w}, x[4] = {0.f, 0.f, 0.f, 0.f}, o[4] = {0.f, 0.f, 0.f, 0.f};
           if (big) {
@@ -348,8 +373,6 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
               if (j == 0) v[0] = t; else if (j == 1) v[1] = t; else if (j == 2) v[2] = t; else v[3] = t;
             }
           }
-          float *dst = C + m * g.ldc + n;
-          const int64_t aux_at = m * g.ld_aux + n;
           if (g.vec_c && n + 4 <= g.N) {
             if (aux_read) {
               const float4 t = *reinterpret_cast<const float4 *>(aux_in + aux_at);
