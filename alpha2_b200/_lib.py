@@ -1,4 +1,5 @@
-"""ctypes binding of libalpha_cuda.so (the C ABI declared in include/alpha_cuda.h).
+"""Binding of libalpha_cuda.so (the C ABI declared in include/alpha_cuda.h): ctypes, and for the entry
+points that take numbers only the compiled callers of hostcall.c under the same names.
 
 This is the Python twin of the FFI stub a TypeScript host would write with bun:ffi.  The
 library is built in-tree by ``python -m alpha2_b200.build``; loading fails loudly when it is
@@ -129,11 +130,13 @@ _OTHER_RESTYPE = {"alpha_last_error": ([], C.c_char_p), "alpha_rng_next": ([C.PO
                   "alpha_rng_gauss": ([C.POINTER(HostRng)], C.c_double)}
 
 _lib = None
+#: device buffer type of hostcall.c, set by load(): Buffer(nbytes) allocates in the library's pool
+Buffer = None
 
 
 def load():
     """Load libalpha_cuda.so and bind every entry point.  Raises if the library is absent."""
-    global _lib
+    global _lib, Buffer
     if _lib is not None:
         return _lib
     if not os.path.exists(SO_PATH):
@@ -149,6 +152,17 @@ def load():
         fn = getattr(L, name)
         fn.argtypes = argtypes
         fn.restype = restype
+    try:
+        from . import _hostcall
+    except ImportError as e:
+        raise AlphaCudaError(f"the compiled callers are missing or do not fit ({e}): build them with "
+                             "`python -m alpha2_b200.build`") from e
+    _hostcall.set_error_class(AlphaCudaError)
+    for name in SIGNATURES:
+        fast = getattr(_hostcall, name, None)
+        if fast is not None:
+            setattr(L, name, fast)
+    Buffer = _hostcall.Buffer
     _lib = L
     return L
 

@@ -31,34 +31,13 @@ _NP = {"f32": np.float32, "i32": np.int32}
 
 
 def _size(shape) -> int:
-    n = 1
-    for d in shape:
-        n *= int(d)
-    return n
+    return math.prod(map(int, shape))
 
 
-class _DeviceBuffer:
+def _DeviceBuffer(nbytes: int):
     """One allocation from the library's caching pool; freed when the last owner lets go."""
-    __slots__ = ("ptr", "nbytes", "__weakref__")
-
-    def __init__(self, nbytes: int):
-        out = C.c_uint64()
-        check(L.load().alpha_alloc(max(int(nbytes), 1), C.byref(out)))
-        self.ptr = out.value
-        self.nbytes = int(nbytes)
-
-    def free(self):
-        if self.ptr:
-            lib = L._lib
-            if lib is not None:
-                lib.alpha_free(self.ptr)
-            self.ptr = 0
-
-    def __del__(self):
-        try:
-            self.free()
-        except Exception:
-            pass
+    L.load()
+    return L.Buffer(int(nbytes))
 
 
 def bf16_to_f32(raw_u16: np.ndarray) -> np.ndarray:
@@ -79,8 +58,8 @@ class TensorData:
     """``{shape, dtype, data}`` (interfaces.ts:31-35) with lazy device residence."""
     __slots__ = ("shape", "dtype", "_buf", "_host", "_released", "__weakref__")
 
-    def __init__(self, shape, dtype: str = "f32", buf: _DeviceBuffer | None = None, host: np.ndarray | None = None):
-        self.shape = tuple(int(d) for d in shape)
+    def __init__(self, shape, dtype: str = "f32", buf=None, host: np.ndarray | None = None):
+        self.shape = tuple(map(int, shape))
         self.dtype = dtype
         self._buf = buf
         self._host = host
@@ -95,7 +74,7 @@ class TensorData:
 
     @property
     def size(self) -> int:
-        return _size(self.shape)
+        return math.prod(self.shape)
 
     @property
     def nbytes(self) -> int:
@@ -177,8 +156,9 @@ class CudaBackend:
 
     # ── helpers ──────────────────────────────────────────────────────────────
     def _new(self, shape, dtype) -> TensorData:
-        shape = tuple(int(d) for d in shape)
-        return TensorData(shape, dtype, _DeviceBuffer(_size(shape) * L.DTYPE_SIZE[dtype]))
+        t = TensorData(shape, dtype)
+        t._buf = L.Buffer(math.prod(t.shape) * L.DTYPE_SIZE[dtype])
+        return t
 
     @staticmethod
     def _code(dtype: str) -> int:
@@ -451,15 +431,18 @@ class CudaBackend:
     # ── matmul family (interfaces.ts:53,111-112) ─────────────────────────────
     def _gemm(self, layout, a, b, M, N, K, lda, ldb, out_dtype=None, epilogue=L.EPI_NONE, aux=None,
               out: TensorData | None = None, accumulate: bool = False, out_shape=None) -> TensorData:
-        if a.dtype != b.dtype:
-            raise AlphaCudaError(f"matmul: dtype mismatch {a.dtype} vs {b.dtype}")
-        out_dtype = out_dtype or a.dtype
+        dtype = a.dtype
+        if dtype != b.dtype:
+            raise AlphaCudaError(f"matmul: dtype mismatch {dtype} vs {b.dtype}")
+        out_dtype = out_dtype or dtype
         if out is None:
             out = self._new(out_shape if out_shape is not None else (M, N), out_dtype)
-        check(self.lib.alpha_gemm(layout, a.ptr, b.ptr, out.ptr, M, N, K, lda, ldb, N, self._code(a.dtype),
-                                  self._code(out_dtype), epilogue, aux.ptr if aux is not None else 0, N,
-                                  1 if accumulate else 0))
-        out.invalidate_host()
+        code = L.DTYPE_CODE
+        status = self.lib.alpha_gemm(layout, a.ptr, b.ptr, out.ptr, M, N, K, lda, ldb, N, code[dtype], code[out_dtype],
+                                     epilogue, aux.ptr if aux is not None else 0, N, 1 if accumulate else 0)
+        if status:
+            check(status)
+        out._host = None
         return out
 
     def matmul(self, a: TensorData, b: TensorData) -> TensorData:
@@ -843,8 +826,9 @@ class CudaBackend:
         E3 = qkv.shape[-1]
         E = E3 // 3
         D = E // H
-        return L.AttnParams(batch=Bn, heads=H, T=T, D=D, q_sb=T * E3, q_sh=D, q_st=E3, o_sb=T * E, o_sh=D, o_st=E,
-                            scale=float(scale), soft_cap=float(softCap), dtype=self._code(qkv.dtype)), E, D
+        # positional, in the order of the fields: batch, heads, T, D, q_sb, q_sh, q_st, o_sb, o_sh, o_st, scale, cap, dtype
+        return L.AttnParams(Bn, H, T, D, T * E3, D, E3, T * E, D, E, float(scale), float(softCap),
+                            L.DTYPE_CODE[qkv.dtype]), E, D
 
     def attentionQkv(self, qkv: TensorData, Bn: int, T: int, H: int, scale: float, softCap: float):
         """Causal multi-head attention reading q, k, v in place from the fused projection
@@ -905,10 +889,10 @@ class CudaBackend:
         """entries: (param, grad, m, v, weightDecay, shadow|None).  One launch for all tensors;
         with clipSumSq the clip coefficient is derived on the device (trainer.ts:1650-1656)."""
         entries = list(entries)
-        arr = (L.AdamWTensor * len(entries))()
-        for i, (p, g, m, v, wd, sh) in enumerate(entries):
-            arr[i] = L.AdamWTensor(p.ptr, g.ptr, m.ptr, v.ptr, sh.ptr if sh is not None else 0, p.size, wd,
-                                   self._code(g.dtype))
+        code = L.DTYPE_CODE
+        arr = (L.AdamWTensor * len(entries))(*[
+            (p.ptr, g.ptr, m.ptr, v.ptr, sh.ptr if sh is not None else 0, p.size, wd, code[g.dtype])
+            for p, g, m, v, wd, sh in entries])
         check(self.lib.alpha_adamw_multi(arr, len(entries), lr, beta1, beta2, eps, bc1, bc2, gradScale,
                                          clipSumSq.ptr if clipSumSq is not None else 0, float(maxNorm)))
         for (p, g, m, v, wd, sh) in entries:

@@ -1,4 +1,4 @@
-"""Builds libalpha_cuda.so in-tree with nvcc for sm_100a.
+"""Builds libalpha_cuda.so in-tree with nvcc for sm_100a, and _hostcall.so, which calls it from Python.
 
     python -m alpha2_b200.build [--force] [--verbose]
 
@@ -12,12 +12,15 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 SO = os.path.join(HERE, "libalpha_cuda.so")
+HOST_SRC = os.path.join(HERE, "hostcall.c")
+HOST_SO = os.path.join(HERE, "_hostcall.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -37,6 +40,47 @@ def _newest_header() -> float:
     hs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + \
         glob.glob(os.path.join(HERE, "..", "include", "*.h"))
     return max(os.path.getmtime(h) for h in hs) if hs else 0.0
+
+
+def hostcall_source() -> str:
+    """hostcall_calls.inc: a METH_FASTCALL function for every entry point that takes numbers only."""
+    import ctypes as C
+
+    from . import _lib as L
+    convert = {C.c_int: ("int", "(int)PyLong_AsLongLong"), C.c_int64: ("int64_t", "PyLong_AsLongLong"),
+               C.c_uint64: ("alpha_buf", "PyLong_AsUnsignedLongLongMask"), C.c_float: ("float", "(float)PyFloat_AsDouble"),
+               C.c_size_t: ("size_t", "PyLong_AsUnsignedLongLongMask")}
+    out, table = [], []
+    for name, args in L.SIGNATURES.items():
+        if not args or any(a not in convert for a in args):
+            continue
+        lines = [f"static PyObject *call_{name}(PyObject *self, PyObject *const *a, Py_ssize_t n) {{",
+                 f'  if (n != {len(args)}) return wrong_count("{name}", {len(args)}, n);']
+        lines += [f"  const {convert[t][0]} v{i} = {convert[t][1]}(a[{i}]);" for i, t in enumerate(args)]
+        lines += ["  if (PyErr_Occurred()) return NULL;", "  int status;", "  Py_BEGIN_ALLOW_THREADS",
+                  f"  status = {name}({', '.join(f'v{i}' for i in range(len(args)))});", "  Py_END_ALLOW_THREADS",
+                  "  return PyLong_FromLong(status);", "}"]
+        out.append("\n".join(lines))
+        table.append(f'  {{"{name}", (PyCFunction)(void (*)(void))call_{name}, METH_FASTCALL, NULL}},')
+    return "\n\n".join(out) + "\n\n#define HOSTCALL_METHODS \\\n" + " \\\n".join(table) + "\n"
+
+
+def build_hostcall(force: bool = False) -> str:
+    inc = os.path.join(OBJ, "hostcall_calls.inc")
+    text = hostcall_source()
+    newest = max(os.path.getmtime(HOST_SRC), _newest_header())
+    same = os.path.exists(inc) and open(inc).read() == text
+    if force or not same or not os.path.exists(HOST_SO) or os.path.getmtime(HOST_SO) < newest:
+        with open(inc, "w") as f:
+            f.write(text)
+        tmp = HOST_SO + ".tmp.%d" % os.getpid()
+        cmd = [os.environ.get("CC", "gcc"), "-O2", "-Wall", "-shared", "-fPIC", "-I", OBJ, "-I", HERE,
+               "-I", sysconfig.get_paths()["include"], HOST_SRC, "-o", tmp]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("gcc failed: %s\n%s\n%s" % (" ".join(cmd), r.stdout, r.stderr))
+        os.replace(tmp, HOST_SO)
+    return HOST_SO
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -71,6 +115,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             raise RuntimeError("link failed: %s\n%s" % (r.stdout, r.stderr))
         os.replace(tmp, SO)
+    build_hostcall(force)
     return SO
 
 

@@ -88,17 +88,11 @@ def next_token(lastLogits: np.ndarray, rng, temperature: float, topk: int, topp:
                 return sampled
     maxVal = float(np.max(logits))                         # :171-195
     probs = np.exp(logits.astype(np.float64) - maxVal).astype(np.float32)
-    sumExp = 0.0
-    for p in probs:
-        sumExp += float(p)
+    # running sums in index order, each rounded to 64 bits like a loop's (ufunc.accumulate adds one by one)
+    sumExp = float(np.add.accumulate(probs.astype(np.float64))[-1])
     probs = (probs.astype(np.float64) / sumExp).astype(np.float32)
-    r = rng.next()
-    cumsum = 0.0
-    for v in range(vocab):
-        cumsum += float(probs[v])
-        if r < cumsum:
-            return v
-    return 0
+    hit = np.nonzero(rng.next() < np.add.accumulate(probs.astype(np.float64)))[0]
+    return int(hit[0]) if hit.size else 0
 
 
 def sample_tokens(config, params, backend, rng, promptTokens, steps: int, temperature: float = 1.0, topk: int = 0,

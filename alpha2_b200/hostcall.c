@@ -1,0 +1,113 @@
+/* Calls of libalpha_cuda.so from Python without ctypes.
+ *
+ * A step of a small model is bound by the host: ctypes takes about 2 microseconds to convert the
+ * arguments of alpha_gemm and another 3 to allocate and free a tensor through Python objects, against
+ * 3 to 5 for the launch itself.  With the callers below the 67 launches of the two-layer byte model's step went
+ * from 768 to 547 microseconds, the 89 of one 124M forward over 200 tokens from 1016 to 884.  Here every entry point that takes numbers only is a METH_FASTCALL
+ * function (generated from the signature table of _lib.py into hostcall_calls.inc, so there is one
+ * table), and the device buffer is a C type that allocates and frees in the library's pool.
+ *
+ * The symbols of the library are resolved at import from the copy that _lib.py has loaded globally.
+ * The GIL is released around every call, as ctypes does.
+ */
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+#include <stddef.h>
+#include <structmember.h>
+
+#include "../include/alpha_cuda.h"
+
+static PyObject *g_error;   /* AlphaCudaError */
+
+static PyObject *wrong_count(const char *name, int want, Py_ssize_t got) {
+  PyErr_Format(PyExc_TypeError, "%s takes %d arguments (%zd given)", name, want, got);
+  return NULL;
+}
+
+#include "hostcall_calls.inc"
+
+typedef struct {
+  PyObject_HEAD
+  unsigned long long ptr;
+  Py_ssize_t nbytes;
+  PyObject *weakrefs;
+} Buffer;
+
+static PyObject *buffer_new(PyTypeObject *type, PyObject *args, PyObject *kwds) {
+  Py_ssize_t nbytes;
+  if (kwds && PyDict_GET_SIZE(kwds)) {
+    PyErr_SetString(PyExc_TypeError, "Buffer takes no keyword arguments");
+    return NULL;
+  }
+  if (!PyArg_ParseTuple(args, "n", &nbytes)) return NULL;
+  Buffer *self = (Buffer *)type->tp_alloc(type, 0);   /* zeroed: nothing to free if the allocation fails */
+  if (!self) return NULL;
+  alpha_buf p = 0;
+  int status;
+  Py_BEGIN_ALLOW_THREADS
+  status = alpha_alloc(nbytes > 0 ? (size_t)nbytes : 1, &p);
+  Py_END_ALLOW_THREADS
+  if (status) {
+    PyErr_SetString(g_error ? g_error : PyExc_RuntimeError, alpha_last_error());
+    Py_DECREF(self);
+    return NULL;
+  }
+  self->ptr = p;
+  self->nbytes = nbytes;
+  return (PyObject *)self;
+}
+
+static void buffer_release(Buffer *self) {
+  if (self->ptr) {
+    alpha_free(self->ptr);
+    self->ptr = 0;
+  }
+}
+
+static void buffer_dealloc(Buffer *self) {
+  if (self->weakrefs) PyObject_ClearWeakRefs((PyObject *)self);
+  buffer_release(self);
+  Py_TYPE(self)->tp_free((PyObject *)self);
+}
+
+static PyObject *buffer_free(PyObject *self, PyObject *unused) {
+  buffer_release((Buffer *)self);
+  Py_RETURN_NONE;
+}
+
+static PyMemberDef buffer_members[] = {{"ptr", T_ULONGLONG, offsetof(Buffer, ptr), READONLY, "device address, 0 once freed"},
+                                       {"nbytes", T_PYSSIZET, offsetof(Buffer, nbytes), READONLY, "size asked for"},
+                                       {NULL}};
+static PyMethodDef buffer_methods[] = {{"free", buffer_free, METH_NOARGS, "Give the memory back to the pool now."}, {NULL}};
+static PyTypeObject BufferType = {
+    PyVarObject_HEAD_INIT(NULL, 0).tp_name = "alpha2_b200._hostcall.Buffer",
+    .tp_basicsize = sizeof(Buffer),
+    .tp_flags = Py_TPFLAGS_DEFAULT,
+    .tp_doc = "One allocation from the library's caching pool; freed when the last owner lets go.",
+    .tp_new = buffer_new,
+    .tp_dealloc = (destructor)buffer_dealloc,
+    .tp_members = buffer_members,
+    .tp_methods = buffer_methods,
+    .tp_weaklistoffset = offsetof(Buffer, weakrefs),
+};
+
+static PyObject *set_error_class(PyObject *self, PyObject *cls) {
+  Py_INCREF(cls);
+  Py_XSETREF(g_error, cls);
+  Py_RETURN_NONE;
+}
+
+static PyMethodDef module_methods[] = {
+    {"set_error_class", set_error_class, METH_O, "The exception that a failed allocation raises."},
+    HOSTCALL_METHODS{NULL}};
+static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hostcall", NULL, -1, module_methods};
+
+PyMODINIT_FUNC PyInit__hostcall(void) {
+  if (PyType_Ready(&BufferType) < 0) return NULL;
+  PyObject *m = PyModule_Create(&module);
+  if (!m || PyModule_AddObjectRef(m, "Buffer", (PyObject *)&BufferType) < 0) {
+    Py_XDECREF(m);
+    return NULL;
+  }
+  return m;
+}

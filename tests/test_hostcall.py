@@ -1,0 +1,123 @@
+"""The compiled callers (hostcall.c) and the sampling sums, on the CPU."""
+import os
+import shutil
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+STUB = r"""
+#include <stdio.h>
+#include <stdint.h>
+typedef uint64_t alpha_buf;
+static char seen[512];
+const char *alpha_last_error(void) { return seen; }
+int alpha_alloc(size_t n, alpha_buf *out) {
+  if (n == 77) { snprintf(seen, sizeof seen, "no room"); return 1; }
+  *out = 4096 + n; snprintf(seen, sizeof seen, "alloc %zu", n); return 0;
+}
+int alpha_free(alpha_buf b) { snprintf(seen, sizeof seen, "free %llu", (unsigned long long)b); return 0; }
+int alpha_gemm(int a, alpha_buf b, alpha_buf c, alpha_buf d, int64_t e, int64_t f, int64_t g, int64_t h, int64_t i,
+               int64_t j, int k, int l, int m, alpha_buf n, int64_t o, int p) {
+  snprintf(seen, sizeof seen, "%d %llu %llu %llu %lld %lld %lld %lld %lld %lld %d %d %d %llu %lld %d", a,
+           (unsigned long long)b, (unsigned long long)c, (unsigned long long)d, (long long)e, (long long)f, (long long)g,
+           (long long)h, (long long)i, (long long)j, k, l, m, (unsigned long long)n, (long long)o, p);
+  return a;
+}
+int alpha_fill(alpha_buf b, int64_t n, float v, int k) { snprintf(seen, sizeof seen, "%llu %lld %.9g %d", (unsigned long long)b, (long long)n, v, k); return 0; }
+"""
+
+CHECK = r"""
+import ctypes, sys
+sys.path.insert(0, sys.argv[2])
+from alpha2_b200 import _lib as L
+L.SO_PATH = sys.argv[1]
+lib = L.load()
+seen = lambda: lib.alpha_last_error().decode()
+for name, args in L.SIGNATURES.items():
+    numbers = all(t in (ctypes.c_int, ctypes.c_int64, ctypes.c_uint64, ctypes.c_float, ctypes.c_size_t) for t in args)
+    assert (type(getattr(lib, name)).__name__ == "builtin_function_or_method") == (numbers and len(args) > 0), name
+a = (-3, 2 ** 64 - 1, 2 ** 40 + 5, 0, -2 ** 62, 2 ** 62, 7, 8, 9, 10, -1, 2 ** 31 - 1, 3, 2 ** 63, -4, 1)
+assert lib.alpha_gemm(*a) == -3 and seen() == " ".join(map(str, a))
+assert lib.alpha_fill(5, 6, 0.1, 2) == 0 and seen() == "5 6 0.100000001 2"
+for wrong in (a[:-1], a + (1,), ("x",) + a[1:], (1.5,) + a[1:]):
+    try:
+        lib.alpha_gemm(*wrong)
+    except TypeError:
+        continue
+    raise SystemExit("accepted %r" % (wrong,))
+b = L.Buffer(100)
+assert (b.ptr, b.nbytes) == (4196, 100)
+b.free()
+assert seen() == "free 4196" and b.ptr == 0
+b.free()                                   # once only
+c = L.Buffer(0)
+assert seen() == "alloc 1"                 # an empty tensor still has an address
+del c
+assert seen() == "free 4097"
+try:
+    L.Buffer(77)
+except L.AlphaCudaError as e:
+    assert str(e) == "no room"
+else:
+    raise SystemExit("a failed allocation went unnoticed")
+assert seen() == "no room"                 # and nothing was freed for it
+print("ok")
+"""
+
+
+@pytest.mark.skipif(shutil.which("gcc") is None, reason="needs gcc")
+def test_compiled_callers_pass_their_arguments_through(tmp_path):
+    from alpha2_b200 import _lib as L
+    have = {"alpha_alloc", "alpha_free", "alpha_gemm", "alpha_fill"}
+    rest = "\n".join(f"int {n}(void) {{ return 0; }}" for n in list(L.SIGNATURES) if n not in have)
+    rest += "\n" + "\n".join(f"void *{n}(void) {{ return 0; }}" for n in L._OTHER_RESTYPE if n != "alpha_last_error")
+    src, so = tmp_path / "stub.c", tmp_path / "stub.so"
+    src.write_text(STUB + rest)
+    subprocess.check_call(["gcc", "-shared", "-fPIC", "-w", "-o", str(so), str(src)])
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", CHECK, str(so), root], capture_output=True, text=True)
+    assert r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+class FixedRng:
+    def __init__(self, x):
+        self.x = x
+
+    def next(self):
+        return self.x
+
+
+def by_loops(row, r, temperature, topk):
+    """The last part of next_token one element at a time."""
+    logits = (row.astype(np.float64) / temperature).astype(np.float32)
+    if 0 < topk < row.size:
+        logits = np.where(logits < np.sort(logits)[::-1][topk - 1], np.float32(-np.inf), logits)
+    probs = np.exp(logits.astype(np.float64) - float(np.max(logits))).astype(np.float32)
+    total = 0.0
+    for p in probs:
+        total += float(p)
+    probs = (probs.astype(np.float64) / total).astype(np.float32)
+    cum = 0.0
+    for v in range(row.size):
+        cum += float(probs[v])
+        if r < cum:
+            return v
+    return 0
+
+
+@pytest.mark.parametrize("vocab", [1, 2, 7, 256, 4096])
+@pytest.mark.parametrize("topk", [0, 5])
+@pytest.mark.filterwarnings("ignore::RuntimeWarning")
+def test_sampling_sums_are_those_of_a_loop(vocab, topk):
+    from alpha2_b200.eval import next_token
+    g = np.random.default_rng(vocab + topk)
+    for i in range(12):
+        row = (g.standard_normal(vocab) * 3).astype(np.float32)
+        if i == 10:
+            row[vocab // 2] = np.nan
+        if i == 11:
+            row[vocab // 2] = -np.inf
+        for r in (0.0, g.random(), np.nextafter(1.0, 0.0)):
+            assert next_token(row, FixedRng(r), 0.7, topk, None) == by_loops(row, r, 0.7, topk)
