@@ -10,7 +10,7 @@
 //
 // Shape of the kernel
 //   * persistent: one CTA per SM walks output tiles (grouped order for L2 reuse);
-//   * pair form (the default for M > 128, N > 128): two CTAs of a cluster share a 256 x 256
+//   * pair form (large products; tc_plan draws the line): two CTAs of a cluster share a 256 x 256
 //     tile through tcgen05 cta_group::2 — each loads its 128 rows of A and 128 of the 256
 //     rows of B, so an SM fetches 32 KB per K step instead of 48 KB for the same tensor-core
 //     work (the single-CTA form is bound by what one SM can pull from L2), 6-stage ring;
@@ -22,8 +22,9 @@
 //   * operands may be K-major or MN-major (the transposed layouts are read in place through
 //     MN-major descriptors, nothing is transposed in memory);
 //   * every CTA issues its own TMA loads (nothing is broadcast between CTAs);
-//   * split-K for the weight-gradient shapes (few output tiles, K = tokens): partial
-//     products go to an fp32 workspace and a second kernel adds them in split order.
+//   * split-K where the output has few tiles (weight gradients, few rows): partial
+//     products go to an fp32 workspace and a second kernel adds them in split order and
+//     applies the epilogue.
 // Algorithmic work: 2*M*N*K flop; bytes (M*K + N*K)*2 + M*N*e_out.
 #include <string.h>
 
@@ -618,39 +619,84 @@ gemm_tc_pair_group2_kernel(const __grid_constant__ GemmTmaps m0, const __grid_co
   gemm_tc_body<256, A_MN, B_MN, true, false, true>(p0, p1);
 }
 
-// C (+)= sum_s ws[s]  — split order is fixed, so the result is reproducible.  ws holds
+// C = epilogue(sum_s ws[s]) (+ C)  — split order is fixed, so the result is reproducible.  ws holds
 // `splits` dense [m_pad, N] fp32 slabs (`slab` elements apart; only the first M rows of each are
-// read); four columns per thread when the rows allow it.
+// read); four columns per thread when the rows allow it.  The epilogue is the unsplit kernel's, on the
+// fp32 sum, its operand and result in C's element type.
+struct SplitkReduceArgs {
+  const float *ws;
+  void *C, *aux;
+  int64_t M, N, ldc, ld_aux, slab;
+  int splits, epilogue, accumulate, vec4;
+};
+
+__device__ __forceinline__ void load4(const float *p, float (&x)[4]) {
+  const float4 t = *reinterpret_cast<const float4 *>(p);
+  x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+}
+__device__ __forceinline__ void load4(const __nv_bfloat16 *p, float (&x)[4]) {
+  const uint2 t = *reinterpret_cast<const uint2 *>(p);
+  f2_unpack(bf16x2_to_f2(t.x), x[0], x[1]);
+  f2_unpack(bf16x2_to_f2(t.y), x[2], x[3]);
+}
+__device__ __forceinline__ void store4(float *p, const float (&x)[4]) {
+  *reinterpret_cast<float4 *>(p) = make_float4(x[0], x[1], x[2], x[3]);
+}
+__device__ __forceinline__ void store4(__nv_bfloat16 *p, const float (&x)[4]) {
+  *reinterpret_cast<uint2 *>(p) = make_uint2(bf16x2_pack(x[0], x[1]), bf16x2_pack(x[2], x[3]));
+}
+
 template <typename OutT>
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ ws, OutT *C, int64_t M, int64_t N,
-                                                            int64_t ldc, int splits, int accumulate, int vec4,
-                                                            int64_t slab) {
-  const int64_t total = M * N;
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitkReduceArgs g) {
+  const int64_t total = g.M * g.N;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   grid_dependency_trigger();
   grid_dependency_wait();  // the slabs come from the GEMM launched just before
-  if (vec4) {
+  const bool reads_aux = g.epilogue == ALPHA_EPI_ADD || g.epilogue == ALPHA_EPI_GELU_BWD;
+  auto finish2 = [&](float &u, float &v, float xu, float xv) {
+    if (g.epilogue == ALPHA_EPI_GELU) {
+      gelu_fast2(u, v);
+    } else if (g.epilogue == ALPHA_EPI_ADD) {
+      u += xu;
+      v += xv;
+    } else if (g.epilogue == ALPHA_EPI_GELU_BWD) {
+      gelu_grad_mul2(u, v, xu, xv);
+    }
+  };
+  if (g.vec4) {
     const int64_t n4 = total / 4;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-      float4 s = reinterpret_cast<const float4 *>(ws)[i];
-      for (int k = 1; k < splits; k++) {
-        const float4 t = reinterpret_cast<const float4 *>(ws + (int64_t)k * slab)[i];
+      float4 s = reinterpret_cast<const float4 *>(g.ws)[i];
+#pragma unroll 4
+      for (int k = 1; k < g.splits; k++) {
+        const float4 t = reinterpret_cast<const float4 *>(g.ws + (int64_t)k * g.slab)[i];
         s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
       }
-      const int64_t e = i * 4, m = e / N, n = e - m * N;
-      OutT *dst = C + m * ldc + n;
-      float o[4] = {s.x, s.y, s.z, s.w};
+      const int64_t e = i * 4, m = e / g.N, n = e - m * g.N;
+      OutT *dst = (OutT *)g.C + m * g.ldc + n, *aux = (OutT *)g.aux + m * g.ld_aux + n;
+      float o[4] = {s.x, s.y, s.z, s.w}, x[4] = {0.f, 0.f, 0.f, 0.f};
+      if (reads_aux) load4(aux, x);
+      if (g.epilogue == ALPHA_EPI_GELU) store4(aux, o);
+      finish2(o[0], o[1], x[0], x[1]);
+      finish2(o[2], o[3], x[2], x[3]);
+      if (g.accumulate) {
+        load4(dst, x);
 #pragma unroll
-      for (int j = 0; j < 4; j++) dst[j] = from_f32<OutT>(accumulate ? to_f32(dst[j]) + o[j] : o[j]);
+        for (int j = 0; j < 4; j++) o[j] = x[j] + o[j];
+      }
+      store4(dst, o);
     }
     return;
   }
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    float s = 0.f;
-    for (int k = 0; k < splits; k++) s += ws[(int64_t)k * slab + i];
-    const int64_t m = i / N, n = i - m * N;
-    OutT *dst = C + m * ldc + n;
-    *dst = from_f32<OutT>(accumulate ? to_f32(*dst) + s : s);
+    float s = 0.f, unused = 0.f;
+    for (int k = 0; k < g.splits; k++) s += g.ws[(int64_t)k * g.slab + i];
+    const int64_t m = i / g.N, n = i - m * g.N;
+    OutT *dst = (OutT *)g.C + m * g.ldc + n, *aux = (OutT *)g.aux + m * g.ld_aux + n;
+    const float x = reads_aux ? to_f32(*aux) : 0.f;
+    if (g.epilogue == ALPHA_EPI_GELU) *aux = from_f32<OutT>(s);
+    finish2(s, unused, x, 0.f);
+    *dst = from_f32<OutT>(g.accumulate ? to_f32(*dst) + s : s);
   }
 }
 
@@ -752,6 +798,54 @@ static int launch_pair_variant(const CUtensorMap &ta, const CUtensorMap &tb, con
   return 0;
 }
 
+// Adds the slabs of a split launch (see splitk_reduce_kernel).
+static int splitk_reduce_launch(SplitkReduceArgs r, int out_dtype) {
+  const size_t quad = 4 * dtype_size(out_dtype);   // bytes of four elements: their alignment in C and aux
+  r.vec4 = r.N % 4 == 0 && r.ldc % 4 == 0 && (uintptr_t)r.C % quad == 0 &&   // ws slabs are 512-byte aligned and dense
+           (r.epilogue == ALPHA_EPI_NONE || (r.ld_aux % 4 == 0 && (uintptr_t)r.aux % quad == 0));
+  const dim3 grid(grid_for(r.M * r.N / (r.vec4 ? 4 : 1) + 1, 256, 8));
+  ALPHA_CUDA(out_dtype == ALPHA_F32
+                 ? launch_overlapped(OVL_SPLITK, splitk_reduce_kernel<float>, grid, dim3(256), 0, r)
+                 : launch_overlapped(OVL_SPLITK, splitk_reduce_kernel<__nv_bfloat16>, grid, dim3(256), 0, r));
+  ALPHA_LAUNCHED();
+  return 0;
+}
+
+// How a product is cut: CTA pairs on 256 x 256 tiles or single CTAs on 128 x bn ones, and K splits.
+// The cut with the least modelled time wins (microseconds, fitted to a sweep of M = 1 ... 16384 over the
+// products of models of width 256 to 768): a launch costs `fixed` and `step` per wave and K step of 64,
+// and splits cost a second launch and the slabs' traffic.  A single CTA with a 128 x 128 tile starts and
+// ends soonest, so it takes what fits in a wave or two; a pair moves the fewest operand bytes per flop and
+// takes the rest, and what the model finds within a tenth (inside a step launches overlap, which hides
+// part of `fixed`: a step of width 384 at 8192 tokens lost 0.8 % without that margin).  E.g. 200 x 768 x 3072 with the residual: 13.0 us by pairs, 10.6 as 128 x 128 in six splits;
+// 2331 x 768 x 768: 12.9 and 9.4; 16384 x 2304 x 768: 40.2 and 65.7.
+struct TcPlan {
+  int pair, bn, splits;
+};
+static TcPlan tc_plan(int64_t M, int64_t N, int64_t kblocks, bool can_split) {
+  static const struct { int pair, bn; double fixed, step; } cuts[3] = {{1, 256, 5.5, 0.37}, {0, 256, 4.8, 0.42}, {0, 128, 3.7, 0.33}};
+  TcPlan best{0, 128, 1};
+  double best_t = 1e30;
+  for (const auto &c : cuts) {
+    if (N <= 128 && c.bn > 128) continue;
+    const int64_t tile_m = c.pair ? 2 * GBM : GBM, slots = c.pair ? g_sm_count / 2 : g_sm_count;
+    const int64_t tiles = ((M + tile_m - 1) / tile_m) * ((N + c.bn - 1) / c.bn);
+    // splits of at least two K steps while the tiles leave the device idle
+    const int64_t max_splits = can_split && tiles < slots ? (kblocks / 2 < 32 ? kblocks / 2 : 32) : 1;
+    for (int64_t sp = 1; sp <= max_splits || sp == 1; sp++) {
+      const int64_t waves = (tiles * sp + slots - 1) / slots, kb = (kblocks + sp - 1) / sp;
+      double t = c.fixed + (double)(waves * kb) * c.step;
+      if (sp > 1) t += 2.6 + (double)(sp + 1) * (double)M * (double)N * 4.0 / 5.0e6;
+      if (c.pair) t *= 0.9;
+      if (t < best_t) {
+        best_t = t;
+        best = TcPlan{c.pair, c.bn, (int)sp};
+      }
+    }
+  }
+  return best;
+}
+
 int gemm_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M, int64_t N, int64_t K, int64_t lda,
                    int64_t ldb, int64_t ldc, int out_dtype, int epilogue, alpha_buf aux, int64_t ld_aux,
                    int accumulate, float *rowdot = nullptr, int rd_T = 0, int rd_H = 0) {
@@ -768,8 +862,10 @@ int gemm_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M,
   ProfScope prof(PROF_GEMM_TC, 2.0 * (double)M * (double)N * (double)K);
   const bool a_mn = layout == ALPHA_GEMM_TN;
   const bool b_mn = layout != ALPHA_GEMM_NT;
-  const int BN = N <= 128 ? 128 : 256;
-  const bool pair = BN == 256 && M > GBM;  // two CTAs per 256 x 256 tile
+  if (epilogue != ALPHA_EPI_NONE) ALPHA_CHECK(aux != 0, "alpha_gemm: epilogue %d needs an aux buffer", epilogue);
+  const TcPlan plan = tc_plan(M, N, (K + GBK - 1) / GBK, epilogue != ALPHA_EPI_ROWDOT);
+  const int BN = plan.bn;
+  const bool pair = plan.pair;  // two CTAs per 256 x 256 tile
   const int tile_m = pair ? 2 * GBM : GBM;
   CUtensorMap ta, tb;
   // A: K-major [M,K] (inner K) or M-major [K,M] (inner M)
@@ -786,22 +882,7 @@ int gemm_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M,
   g.kblocks = (int)((K + GBK - 1) / GBK);
   g.err = tc_error_word();
   const int tiles = g.tiles_m * g.tiles_n;
-  // Split-K when the output has too few tiles to fill the device: pick the split count that
-  // minimises (waves of tiles) x (K steps per tile + per-tile overhead) + the cost of adding
-  // the fp32 partial slabs, all in units of one K step of one tile walker (~0.5 us).
-  const int slots = pair ? g_sm_count / 2 : g_sm_count;
-  int splits = 1;
-  if (epilogue == ALPHA_EPI_NONE && tiles < slots && g.kblocks >= 16) {
-    const int max_s = g.kblocks / 8 < 32 ? g.kblocks / 8 : 32;
-    double best = 1e30;
-    for (int sp = 1; sp <= max_s; sp++) {
-      const int waves = (tiles * sp + slots - 1) / slots;
-      const int kb = (g.kblocks + sp - 1) / sp;
-      double t = (double)waves * (kb + 3);
-      if (sp > 1) t += (double)(sp + 1) * (double)M * (double)N * 4.0 / 5.0e12 / 0.5e-6;
-      if (t < best) { best = t; splits = sp; }
-    }
-  }
+  int splits = plan.splits;
   g.kb_per_split = (g.kblocks + splits - 1) / splits;
   splits = (g.kblocks + g.kb_per_split - 1) / g.kb_per_split;  // drop empty splits
   g.splits = splits;
@@ -826,7 +907,6 @@ int gemm_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M,
     g.C = ptr<void>(C); g.ldc = ldc; g.out_f32 = out_dtype == ALPHA_F32;
     g.epilogue = epilogue; g.accumulate = accumulate;
     g.aux_in = ptr<void>(aux); g.aux_out = ptr<void>(aux); g.ld_aux = ld_aux;
-    if (epilogue != ALPHA_EPI_NONE) ALPHA_CHECK(aux != 0, "alpha_gemm: epilogue %d needs an aux buffer", epilogue);
   }
   // Outputs leave through shared memory + TMA stores when the layout allows a tensor map
   // (16-byte aligned base and rows) and nothing has to be read back from C.
@@ -870,19 +950,9 @@ int gemm_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M,
   rc = BN == 256 ? GEMM_VARIANT(256) : GEMM_VARIANT(128);
 #undef GEMM_VARIANT
   }
-  if (rc == 0 && splits > 1) {
-    const int vec4 = (N % 4 == 0) ? 1 : 0;   // ws slabs are 512-byte aligned and dense
-    const int rgrid = grid_for(M * N / (vec4 ? 4 : 1) + 1, 256, 8);
-    cudaError_t e;
-    if (out_dtype == ALPHA_F32)
-      e = launch_overlapped(OVL_SPLITK, splitk_reduce_kernel<float>, dim3(rgrid), dim3(256), 0, (const float *)ws, ptr<float>(C), M,
-                            N, ldc, splits, accumulate, vec4, (int64_t)g.m_pad * N);
-    else
-      e = launch_overlapped(OVL_SPLITK, splitk_reduce_kernel<__nv_bfloat16>, dim3(rgrid), dim3(256), 0, (const float *)ws,
-                            ptr<__nv_bfloat16>(C), M, N, ldc, splits, accumulate, vec4, (int64_t)g.m_pad * N);
-    if (e != cudaSuccess) rc = set_error("split-K reduce launch -> %s", cudaGetErrorString(e));
-    g_launches++;
-  }
+  if (rc == 0 && splits > 1)
+    rc = splitk_reduce_launch({(const float *)ws, ptr<void>(C), ptr<void>(aux), M, N, ldc, ld_aux, (int64_t)g.m_pad * N,
+                               splits, epilogue, accumulate, 0}, out_dtype);
   if (ws) pool_free(ws);
   return rc;
 }
@@ -984,7 +1054,7 @@ static int gemm_tn_pair_launch(const TnProblem &q0, const TnProblem &q1, int64_t
   }
   const int total = (int)(t0 * g0.splits + t1 * g1.splits);
   const int n = total < max_pairs ? total : max_pairs;
-  cudaError_t e = launch_overlapped(OVL_GEMM, gemm_tc_pair_group2_kernel<true, true>, dim3(2 * n), dim3(L::THREADS), L::DYN, m0,
+  const cudaError_t e = launch_overlapped(OVL_GEMM, gemm_tc_pair_group2_kernel<true, true>, dim3(2 * n), dim3(L::THREADS), L::DYN, m0,
                                     m1, g0, g1);
   int rc = 0;
   if (e != cudaSuccess) rc = set_error("alpha_gemm_tn_pair: launch -> %s", cudaGetErrorString(e));
@@ -994,12 +1064,9 @@ static int gemm_tn_pair_launch(const TnProblem &q0, const TnProblem &q1, int64_t
   void *wss[2] = {ws0, ws1};
   for (int i = 0; i < 2 && rc == 0; i++) {
     if (gs[i]->splits <= 1) continue;
-    const int rgrid = grid_for(qs[i]->M * qs[i]->N / 4 + 1, 256, 8);
-    e = launch_overlapped(OVL_SPLITK, splitk_reduce_kernel<float>, dim3(rgrid), dim3(256), 0, (const float *)wss[i],
-                          ptr<float>(qs[i]->C), qs[i]->M, qs[i]->N, qs[i]->ldc, gs[i]->splits, qs[i]->accumulate, 1,
-                          (int64_t)gs[i]->m_pad * qs[i]->N);
-    if (e != cudaSuccess) rc = set_error("alpha_gemm_tn_pair: reduce launch -> %s", cudaGetErrorString(e));
-    else g_launches++;
+    rc = splitk_reduce_launch({(const float *)wss[i], ptr<void>(qs[i]->C), nullptr, qs[i]->M, qs[i]->N, qs[i]->ldc, 0,
+                               (int64_t)gs[i]->m_pad * qs[i]->N, gs[i]->splits, ALPHA_EPI_NONE, qs[i]->accumulate, 0},
+                              ALPHA_F32);
   }
   if (ws0) pool_free(ws0);
   if (ws1) pool_free(ws1);

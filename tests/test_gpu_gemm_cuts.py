@@ -1,0 +1,62 @@
+"""The bf16 GEMM over the cuts that its cost model chooses (single CTAs with 128 x 128 and 128 x 256 tiles, CTA pairs,
+K splits with the epilogue behind the sum) against float64 on the rounded operands.
+
+Bound: fp32 accumulation in any order, 2*K*u*sum|a||b| with u = 2^-24 (truncating adds), then one rounding of the
+result (and of the pre-activation that GELU' reads) to bf16, 2^-8; tanh.approx is good to 2^-10.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def B():
+    from alpha2_b200.backend import CudaBackend
+    b = CudaBackend(0)
+    yield b
+    b.checkAsyncError()
+
+
+def rounded(x):
+    from alpha2_b200.backend import bf16_to_f32, f32_to_bf16_bits
+    return bf16_to_f32(f32_to_bf16_bits(x.astype(np.float32))).reshape(x.shape).astype(np.float64)
+
+
+@pytest.mark.parametrize("layout", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K", [(1, 136, 768), (8, 256, 4096), (129, 257, 64), (200, 768, 3072), (130, 1160, 136),
+                                   (777, 136, 1536), (1030, 520, 200), (2336, 776, 768)])
+@pytest.mark.parametrize("epilogue,accumulate,out", [(0, 0, "bf16"), (0, 1, "f32"), (1, 0, "bf16"), (2, 0, "bf16"),
+                                                     (3, 0, "bf16")])
+def test_against_64_bits(B, layout, M, N, K, epilogue, accumulate, out):
+    from alpha2_b200 import _lib as L
+    from alpha2_b200._lib import check
+    ld = lambda n: (n + 7) // 8 * 8                    # rows of 16 bytes, as tensor maps want them
+    g = np.random.default_rng(M + N + K)
+    a, b = rounded(g.standard_normal((M, K)) * 0.1), rounded(g.standard_normal((K, N)))
+    x, c0 = rounded(g.standard_normal((M, N))), rounded(g.standard_normal((M, N)))
+
+    def up(v, dtype):
+        p = np.zeros((v.shape[0], ld(v.shape[1])), np.float32)
+        p[:, :v.shape[1]] = v
+        return B.upload(p, dtype)
+
+    sa, sb = (a.T if layout == 2 else a), (b.T if layout == 0 else b)
+    A, Bm, X, C = up(sa, "bf16"), up(sb, "bf16"), up(x, out), up(c0, out)
+    check(B.lib.alpha_gemm(layout, A.ptr, Bm.ptr, C.ptr, M, N, K, ld(sa.shape[1]), ld(sb.shape[1]), ld(N), L.BF16,
+                           L.DTYPE_CODE[out], epilogue, X.ptr if epilogue else 0, ld(N), accumulate))
+    C.invalidate_host()
+    got = np.array(C.data, np.float64)[:, :N]
+    r = a @ b
+    gelu = lambda t: 0.5 * t * (1 + np.tanh(0.7978845608028654 * (t + 0.044715 * t ** 3)))
+    th = np.tanh(0.7978845608028654 * (x + 0.044715 * x ** 3))
+    slope = 0.5 * (1 + th) + 0.5 * x * (1 - th ** 2) * 0.7978845608028654 * (1 + 3 * 0.044715 * x ** 2)
+    want = [r, gelu(r), r + x, r * slope][epilogue] + accumulate * c0
+    err = 1.13 * 2 * K * 2.0 ** -24 * (np.abs(a) @ np.abs(b)) + (2.0 ** -8 if out == "bf16" else 2.0 ** -22) * np.abs(want)
+    if epilogue in (1, 3):
+        err = err + 2.0 ** -10 * (np.abs(r) * (1 + np.abs(x) * 2 if epilogue == 3 else 1))
+    assert np.all(np.abs(got - want) <= err + 1e-6)
+    if epilogue == 1:
+        X.invalidate_host()
+        pre = np.array(X.data, np.float64)[:, :N]
+        assert np.all(np.abs(pre - r) <= 2 * K * 2.0 ** -24 * (np.abs(a) @ np.abs(b)) + 2.0 ** -8 * np.abs(r) + 1e-6)
