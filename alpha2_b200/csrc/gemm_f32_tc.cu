@@ -11,23 +11,25 @@
 // sum longer than 64 terms.  Error against 64 bits: tests/test_gpu_gemm_f32.py.
 //
 // Shape of the kernel: persistent, one CTA per SM, tile 128 x BN x 64, 16 warps (128 registers each):
-//   warps 0-7   operands: 16-byte global loads (both contiguity directions, coalesced), split in
-//               registers, written as three 128B-swizzled bf16 planes per operand.  The loads of
-//               the next K step are issued as soon as a register has been split.
+//   warps 0-7   operands.  A: 16-byte global loads (both contiguity directions, coalesced) go to shared
+//               memory as they are and come back one row per lane, are split and stored in tensor memory,
+//               from where the MMAs take their left operand: a tile of both operands in shared memory is
+//               read at 64 bytes a clock, which held 128 x 128 MMAs at half of their rate.  B: split in
+//               registers into three 128B-swizzled bf16 planes, or (SPLIT_B) brought by TMA from planes that
+//               f3_split_kernel made.  The next K step's loads are issued as soon as registers are free.
 //   warps 8-15  accumulation: tensor memory -> registers after every K step (two accumulators
 //               alternate), epilogue at the end of the tile through shared memory, so that rows
 //               leave in 128-byte segments.  Warp 8 also issues the MMAs (one elected lane), a K step
 //               ahead of the one whose sums it is about to read.
-// The split happens in the kernel: done in a pass of its own it would read 4 and write 6 bytes per
-// element and operand, which costs a third of the GEMM's own time at K = 384.
 //
 // Infinities: inf splits into inf and NaN terms, and |x| >= 2^127 may round up to inf.  The operand
 // warps flag such a tile, and its elements that came out non-finite are recomputed with an fmaf
 // chain in K order.  NaN operands need nothing: the result is NaN either way.
 //
-// Measured on a B200: 8192 x 4096 x 384 in 199 us (130 TFLOP/s), 16384 x 768 x 256 in 64 us (100); an
-// FMA-pipe kernel with 4 x 4 outputs per thread ran such products at 9 to 15 TFLOP/s.  Bound by the operand
-// warps (splitting and the loads it waits for), not by the tensor core.
+// Measured on a B200: 8192 x 4096 x 384 in 155 us (166 TFLOP/s), 16384 x 768 x 256 in 53 us (123); with both
+// operands in shared memory and B always split here 199 and 64 us; an FMA-pipe kernel with 4 x 4 outputs per
+// thread ran such products at 9 to 15 TFLOP/s.  Bound by the operand warps and, at small K, by the epilogue that
+// the next tile's MMAs overlap with only two K steps deep.
 #include <string.h>
 
 #include "tc_common.cuh"
@@ -35,6 +37,22 @@
 namespace alpha {
 
 using namespace tc;
+
+// D[tmem] (+)= A[tmem] * B[smem desc]; A: one row per lane, two bf16 of consecutive k per column.  ONE thread.
+__device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
 
 struct GemmF32TcArgs {
   const float *A, *B;
@@ -48,6 +66,8 @@ struct GemmF32TcArgs {
   int tiles_m, tiles_n, splits, kb_per_split, kblocks, batch;
   int epilogue, accumulate;
   int vec_a, vec_b, vec_c;   // 16-byte accesses are legal for A / B / (C and aux)
+  const uint32_t *b_big;     // SPLIT_B: a flag per block of the kernel that split B
+  int n_b_big;
   uint32_t *err;
 };
 
@@ -58,12 +78,15 @@ constexpr int F3_FLAGS = 8;   // ring of per-tile "holds an infinity" tags
 
 template <int BN>
 struct F3Layout {
-  static constexpr int A_PLANE = F3_BM * F3_BK * 2, B_PLANE = BN * F3_BK * 2;
-  static constexpr int STAGE = 3 * (A_PLANE + B_PLANE);
-  static constexpr int EPI_OFF = F3_STAGES * STAGE;
+  static constexpr int B_PLANE = BN * F3_BK * 2, STAGE = 3 * B_PLANE;
+  static constexpr int RAW = F3_BM * F3_BK * 4;                    // a tile of A as it comes, fp32; two of them
+  static constexpr int RAW_OFF = F3_STAGES * STAGE;
+  static constexpr int EPI_OFF = RAW_OFF + 2 * RAW;
   static constexpr int BAR_OFF = EPI_OFF + F3_ACC_WARPS * 4096;
-  static constexpr int TOTAL = BAR_OFF + 8 * (2 * F3_STAGES + 4) + 8 + 4 * F3_FLAGS;
+  static constexpr int TOTAL = BAR_OFF + 8 * (2 * F3_STAGES + 6) + 8 + 4 * F3_FLAGS;
   static constexpr int DYN = TOTAL + 1024;   // slack to align the base to 1024 B
+  // tensor memory: two accumulators, then per stage the three planes of A (two k per 32-bit column)
+  static constexpr int A_COL = 2 * BN, A_PLANE_COLS = F3_BK / 2, A_STAGE_COLS = 3 * A_PLANE_COLS, TMEM_COLS = 512;
 };
 
 // x = h + m + l for a pair; each result holds the pair's two bf16 terms
@@ -121,6 +144,20 @@ struct F3Operand {
       r[i] = v;
     }
   }
+  // The tile as it is, for A: K-major rows of 64 k whose 16-byte chunks are swizzled by the row modulo 8 (rows
+  // are read back one per lane), MN-major lines of ROWS elements per k.  Returns as store() does.
+  __device__ __forceinline__ bool store_raw(uint8_t *raw, int tid) const {
+    const int row = row_of(tid, 0), k = k_of(tid, 0);
+    raw += MN ? k * (ROWS * 4) + row * 4 : row * (F3_BK * 4) + (((k >> 2) ^ (row & 7)) << 4);
+    constexpr int PASS = MN ? (1024 / ROWS) * ROWS * 4 : 16 * F3_BK * 4;
+    float top = 0.f;
+#pragma unroll
+    for (int i = 0; i < PASSES; i++) {
+      *reinterpret_cast<float4 *>(raw + i * PASS) = r[i];
+      top = fmax3(top, fmaxf(fabsf(r[i].x), fabsf(r[i].y)), fmaxf(fabsf(r[i].z), fabsf(r[i].w)));
+    }
+    return top >= 1.7014118346046923e38f;   // 2^127; a NaN beside it does not hide it (max drops NaN)
+  }
   // Returns whether the thread's elements hold an infinity or a value from 2^127 on.
   __device__ __forceinline__ bool store(uint8_t *planes, int tid) const {
     // K-major: rows of 64 k (128 bytes); MN-major: atoms of 64 rows, per atom one 128-byte line per k.  The
@@ -141,9 +178,24 @@ struct F3Operand {
       *reinterpret_cast<uint2 *>(planes + 2 * PLANE + i * PASS) = l;
       top = fmax3(top, fmaxf(fabsf(r[i].x), fabsf(r[i].y)), fmaxf(fabsf(r[i].z), fabsf(r[i].w)));
     }
-    return top >= 1.7014118346046923e38f;   // 2^127; a NaN beside it does not hide it (max drops NaN)
+    return top >= 1.7014118346046923e38f;
   }
 };
+
+// Sixteen consecutive k of one row from a raw tile.
+template <bool MN>
+__device__ __forceinline__ void f3_read_row(const uint8_t *raw, int row, int k0, float (&x)[16]) {
+  if (MN) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) x[i] = *reinterpret_cast<const float *>(raw + (k0 + i) * (F3_BM * 4) + row * 4);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const float4 t = *reinterpret_cast<const float4 *>(raw + row * (F3_BK * 4) + ((((k0 >> 2) + c) ^ (row & 7)) << 4));
+      x[4 * c] = t.x; x[4 * c + 1] = t.y; x[4 * c + 2] = t.z; x[4 * c + 3] = t.w;
+    }
+  }
+}
 
 __device__ __forceinline__ void f3_tile(const GemmF32TcArgs &g, int unit, int &z, int &split, int &mt, int &nt) {
   const int per = g.tiles_m * g.tiles_n;
@@ -165,8 +217,10 @@ __device__ __forceinline__ float f3_finish(int epilogue, float v, float aux) {
   return v;
 }
 
-template <bool A_MN, bool B_MN, int BN>
-__global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF32TcArgs g) {
+// SPLIT_B: B was split by f3_split_kernel and its planes arrive by TMA; the operand warps split A only.
+template <bool A_MN, bool B_MN, int BN, bool SPLIT_B>
+__global__ void __launch_bounds__(F3_THREADS, 1)
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const GemmF32TcArgs g) {
   using L = F3Layout<BN>;
   extern __shared__ uint8_t f3_smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)f3_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -175,21 +229,23 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
   auto empty_bar = [&](int s) { return bar + 8u * (F3_STAGES + s); };
   auto tfull_bar = [&](int s) { return bar + 8u * (2 * F3_STAGES + s); };
   auto tempty_bar = [&](int s) { return bar + 8u * (2 * F3_STAGES + 2 + s); };
-  uint32_t *tmem_slot = (uint32_t *)(smem + L::BAR_OFF + 8 * (2 * F3_STAGES + 4));
+  auto raw_bar = [&](int s) { return bar + 8u * (2 * F3_STAGES + 4 + s); };
+  uint32_t *tmem_slot = (uint32_t *)(smem + L::BAR_OFF + 8 * (2 * F3_STAGES + 6));
   volatile uint32_t *abort_flag = (volatile uint32_t *)(tmem_slot + 1);
   volatile uint32_t *big_tag = (volatile uint32_t *)(tmem_slot + 2);   // [F3_FLAGS]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int MMA_WARP = F3_OP_WARPS;
-  constexpr uint32_t TMEM_COLS = 2 * BN;
+  constexpr uint32_t TMEM_COLS = L::TMEM_COLS;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < F3_STAGES; s++) {
-      mbar_init(full_bar(s), F3_OP_WARPS);
+      mbar_init(full_bar(s), F3_OP_WARPS + (SPLIT_B ? 1 : 0));   // the TMA's own arrival
       mbar_init(empty_bar(s), 1);
     }
     for (int s = 0; s < 2; s++) {
       mbar_init(tfull_bar(s), 1);
       mbar_init(tempty_bar(s), F3_ACC_WARPS);
+      mbar_init(raw_bar(s), F3_OP_WARPS);
     }
     *abort_flag = 0;
     for (int i = 0; i < F3_FLAGS; i++) big_tag[i] = 0;
@@ -212,7 +268,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
     // ── operands: global -> registers -> three bf16 planes ────────────────────────────────
     const int tid = threadIdx.x;
     F3Operand<A_MN, F3_BM> a;
-    F3Operand<B_MN, BN> b;
+    F3Operand<B_MN, BN> b;   // not used with SPLIT_B
     int unit = blockIdx.x, z, split, mt, nt, kb = 0, kb1 = 0;
     auto enter = [&]() {   // coordinates of `unit`
       f3_tile(g, unit, z, split, mt, nt);
@@ -221,32 +277,73 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
     };
     auto load_a = [&]() { a.load(g.A + z * g.batch_a, g.lda, mt * F3_BM, g.M, kb * F3_BK, g.K, g.vec_a, tid); };
     auto load_b = [&]() { b.load(g.B + z * g.batch_b, g.ldb, nt * BN, g.N, kb * F3_BK, g.K, g.vec_b, tid); };
+    if (SPLIT_B && warp == 0 && elect_one()) tma_prefetch_desc(&tmap_b);
     if (unit < units) {
       enter();
       load_a();
-      load_b();
+      if (!SPLIT_B) load_b();
     }
-    int stage = 0;
-    uint32_t phase = 0, it = 0;   // it: tiles of this CTA so far
+    // this thread's row of A in tensor memory, and the half of the K step that it splits
+    const int row = (warp & 3) * 32 + lane, k_half = (warp >> 2) * (F3_BK / 2);
+    const uint32_t a_tmem = tmem_base + L::A_COL + ((uint32_t)((warp & 3) * 32) << 16) + k_half / 2;
+    int stage = 0, rb = 0;
+    uint32_t phase = 0, raw_phase = 0, it = 0;   // it: tiles of this CTA so far
     while (unit < units) {
-      if (!mbar_wait(empty_bar(stage), phase ^ 1, abort_flag)) break;
-      uint8_t *st = smem + stage * L::STAGE;
-      // split and store this step; each operand's registers then take the next step's loads
+      // this step's tile of A goes to shared memory as it is, and the registers take the next step's loads
+      uint8_t *st = smem + stage * L::STAGE, *raw = smem + L::RAW_OFF + rb * L::RAW;
       const uint32_t it_now = it;
+      const int b_k = kb * F3_BK, b_n = nt * BN;
       if (++kb == kb1) {
         unit += gridDim.x;
         it++;
         if (unit < units) enter();
       }
-      bool big = a.store(st, tid);
+      bool big = a.store_raw(raw, tid);
       if (unit < units) load_a();
-      big |= b.store(st + 3 * L::A_PLANE, tid);
-      if (unit < units) load_b();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(raw_bar(rb));
+      if (!mbar_wait(empty_bar(stage), phase ^ 1, abort_flag)) break;   // the MMAs that read this stage are done
+      tc_fence_after();
+      if (SPLIT_B) {
+        if (warp == 0 && elect_one()) {
+          mbar_expect_tx(full_bar(stage), 3 * L::B_PLANE);
+#pragma unroll
+          for (int p = 0; p < 3; p++) {
+            if (B_MN) {
+#pragma unroll
+              for (int i = 0; i < BN / 64; i++)
+                tma_load_3d(smem_u32(st) + p * L::B_PLANE + i * 8192, &tmap_b, full_bar(stage), b_n + i * 64, b_k, p);
+            } else {
+              tma_load_3d(smem_u32(st) + p * L::B_PLANE, &tmap_b, full_bar(stage), b_k, b_n, p);
+            }
+          }
+        }
+        __syncwarp();
+      } else {
+        big |= b.store(st, tid);
+        if (unit < units) load_b();
+      }
       if (big) big_tag[it_now % F3_FLAGS] = it_now + 1;
-      fence_proxy_async();
+      // rows of A: shared memory -> three terms -> tensor memory
+      if (!mbar_wait(raw_bar(rb), raw_phase, abort_flag)) break;
+#pragma unroll
+      for (int c = 0; c < F3_BK / 2; c += 16) {
+        float x[16];
+        f3_read_row<A_MN>(raw, row, k_half + c, x);
+        uint32_t t[3][8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) split3(x[2 * i], x[2 * i + 1], t[0][i], t[1][i], t[2][i]);
+#pragma unroll
+        for (int p = 0; p < 3; p++) tmem_st_32x8(a_tmem + stage * L::A_STAGE_COLS + p * L::A_PLANE_COLS + c / 2, t[p]);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      if (!SPLIT_B) fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(full_bar(stage));
       if (++stage == F3_STAGES) { stage = 0; phase ^= 1; }
+      rb ^= 1;
+      if (rb == 0) raw_phase ^= 1;
     }
   } else {
     // ── accumulation and epilogue: 32 rows (TMEM lane quadrant) x BN/2 columns per warp ───
@@ -268,20 +365,19 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
       if (!mbar_wait(tempty_bar(i_acc), i_acc_phase ^ 1, abort_flag) || !mbar_wait(full_bar(i_stage), i_phase, abort_flag))
         return false;
       tc_fence_after();
-      constexpr uint32_t idesc = make_idesc_bf16(F3_BM, BN, A_MN, B_MN);
+      constexpr uint32_t idesc = make_idesc_bf16(F3_BM, BN, false, B_MN);
       // smallest products first; plane 0 = h, 1 = m, 2 = l
       constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
-      const uint32_t a_s = smem_u32(smem) + i_stage * L::STAGE, b_s = a_s + 3 * L::A_PLANE;
-      const uint32_t d = tmem_base + i_acc * BN;
-      const uint64_t ad = A_MN ? make_smem_desc(a_s, 8192, 1024) : make_smem_desc(a_s, 16, 1024);
+      const uint32_t b_s = smem_u32(smem) + i_stage * L::STAGE, d = tmem_base + i_acc * BN;
+      const uint32_t a_t = tmem_base + L::A_COL + i_stage * L::A_STAGE_COLS;
       const uint64_t bd = B_MN ? make_smem_desc(b_s, 8192, 1024) : make_smem_desc(b_s, 16, 1024);
       if (elect_one()) {
 #pragma unroll
         for (int p = 0; p < 6; p++) {
 #pragma unroll
           for (int k = 0; k < F3_BK / 16; k++)
-            mma_bf16_ss(d, ad + ((PA[p] * L::A_PLANE + k * (A_MN ? 2048 : 32)) >> 4),
-                        bd + ((PB[p] * L::B_PLANE + k * (B_MN ? 2048 : 32)) >> 4), idesc, (p | k) ? 1u : 0u);
+            mma_bf16_ts(d, a_t + PA[p] * L::A_PLANE_COLS + k * 8, bd + ((PB[p] * L::B_PLANE + k * (B_MN ? 2048 : 32)) >> 4),
+                        idesc, (p | k) ? 1u : 0u);
         }
         mma_commit(empty_bar(i_stage));
         mma_commit(tfull_bar(i_acc));
@@ -297,6 +393,11 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
       return true;
     };
     if (ew == 0) ok = issue_next();
+    bool b_big = false;
+    if (SPLIT_B) {
+      for (int i = lane; i < g.n_b_big; i += 32) b_big |= g.b_big[i] != 0;
+      b_big = __any_sync(0xffffffffu, b_big);
+    }
     for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x, it++) {
       int z, split, mt, nt;
       f3_tile(g, unit, z, split, mt, nt);
@@ -325,7 +426,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
       }
       if (!ok) break;
       const int m_base = mt * F3_BM + quad * 32, n_base = nt * BN + half * NC;
-      const bool big = big_tag[it % F3_FLAGS] == it + 1;
+      const bool big = b_big || big_tag[it % F3_FLAGS] == it + 1;
       float *C = g.C + split * g.split_c + z * g.batch_c;
       const float *aux_in = g.aux_in;
       const bool plain = g.epilogue == ALPHA_EPI_NONE && !g.accumulate;
@@ -354,49 +455,53 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
           __syncwarp();
           continue;
         }
+        if (g.vec_c && n + 4 <= g.N && !big && !(aux_read && g.accumulate)) {
+          // four rows' operands (the residual, the pre-activation, or C itself) are on the way together; a row past
+          // the end reads the last one
+          const float *src = aux_read ? aux_in + aux_at : dst;
+          const int64_t src_ld = aux_read ? g.ld_aux : g.ldc;
 #pragma unroll 1
-        for (int rr = lane >> 3; rr < rows; rr += 4, dst += 4 * g.ldc, aux_at += 4 * g.ld_aux) {
-          if (n >= g.N) continue;
-          const int64_t m = m_base + rr;
-          const float4 s4 = *reinterpret_cast<const float4 *>(stg + rr * 32 + ((q ^ (rr & 7)) << 2));
-          float v[4] = {s4.x, s4.y, s4.z, s4.w}, x[4] = {0.f, 0.f, 0.f, 0.f}, o[4] = {0.f, 0.f, 0.f, 0.f};
-          if (big) {
-            const int k_end = min(g.K, (kb0 + n_kb) * F3_BK);
-            const float *A = g.A + z * g.batch_a, *B = g.B + z * g.batch_b;
-#pragma unroll 1
-            for (int j = 0; j < 4; j++) {
-              const float had = j == 0 ? v[0] : j == 1 ? v[1] : j == 2 ? v[2] : v[3];
-              if (n + j >= g.N || isfinite(had)) continue;
-              float t = 0.f;
-              for (int k = kb0 * F3_BK; k < k_end; k++)
-                t = fmaf(A_MN ? A[k * g.lda + m] : A[m * g.lda + k], B_MN ? B[k * g.ldb + n + j] : B[(n + j) * g.ldb + k], t);
-              if (j == 0) v[0] = t; else if (j == 1) v[1] = t; else if (j == 2) v[2] = t; else v[3] = t;
+          for (int r0 = lane >> 3; r0 < 32; r0 += 16) {
+            float4 x[4] = {};
+            if (aux_read || g.accumulate) {
+#pragma unroll
+              for (int i = 0; i < 4; i++)
+                x[i] = *reinterpret_cast<const float4 *>(src + (min(r0 + 4 * i, rows - 1) - (lane >> 3)) * src_ld);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const int rr = r0 + 4 * i, down = rr - (lane >> 3);
+              if (rr >= rows) continue;
+              float4 v = *reinterpret_cast<const float4 *>(stg + rr * 32 + ((q ^ (rr & 7)) << 2));
+              if (g.epilogue == ALPHA_EPI_GELU) *reinterpret_cast<float4 *>(g.aux_out + aux_at + down * g.ld_aux) = v;
+              v.x = f3_finish(g.epilogue, v.x, x[i].x);
+              v.y = f3_finish(g.epilogue, v.y, x[i].y);
+              v.z = f3_finish(g.epilogue, v.z, x[i].z);
+              v.w = f3_finish(g.epilogue, v.w, x[i].w);
+              if (g.accumulate) v = make_float4(x[i].x + v.x, x[i].y + v.y, x[i].z + v.z, x[i].w + v.w);
+              *reinterpret_cast<float4 *>(dst + down * g.ldc) = v;
             }
           }
-          if (g.vec_c && n + 4 <= g.N) {
-            if (aux_read) {
-              const float4 t = *reinterpret_cast<const float4 *>(aux_in + aux_at);
-              x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+          __syncwarp();
+          continue;
+        }
+#pragma unroll 1
+        for (int rr = lane >> 3; rr < rows; rr += 4, dst += 4 * g.ldc, aux_at += 4 * g.ld_aux) {
+          const int64_t m = m_base + rr;
+          const float4 s4 = *reinterpret_cast<const float4 *>(stg + rr * 32 + ((q ^ (rr & 7)) << 2));
+#pragma unroll 1
+          for (int j = 0; j < 4 && n + j < g.N; j++) {
+            float v = j == 0 ? s4.x : j == 1 ? s4.y : j == 2 ? s4.z : s4.w;
+            if (big && !isfinite(v)) {
+              const float *A = g.A + z * g.batch_a, *B = g.B + z * g.batch_b;
+              const int k_end = min(g.K, (kb0 + n_kb) * F3_BK);
+              v = 0.f;
+              for (int k = kb0 * F3_BK; k < k_end; k++)
+                v = fmaf(A_MN ? A[k * g.lda + m] : A[m * g.lda + k], B_MN ? B[k * g.ldb + n + j] : B[(n + j) * g.ldb + k], v);
             }
-            if (g.accumulate) {
-              const float4 t = *reinterpret_cast<const float4 *>(dst);
-              o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
-            }
-            if (g.epilogue == ALPHA_EPI_GELU) *reinterpret_cast<float4 *>(g.aux_out + aux_at) = make_float4(v[0], v[1], v[2], v[3]);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-              v[j] = f3_finish(g.epilogue, v[j], x[j]);
-              if (g.accumulate) v[j] = o[j] + v[j];
-            }
-            *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-              if (n + j >= g.N) continue;
-              if (g.epilogue == ALPHA_EPI_GELU) g.aux_out[aux_at + j] = v[j];
-              const float y = f3_finish(g.epilogue, v[j], aux_read ? aux_in[aux_at + j] : 0.f);
-              dst[j] = g.accumulate ? dst[j] + y : y;
-            }
+            if (g.epilogue == ALPHA_EPI_GELU) g.aux_out[aux_at + j] = v;
+            v = f3_finish(g.epilogue, v, aux_read ? aux_in[aux_at + j] : 0.f);
+            dst[j] = g.accumulate ? dst[j] + v : v;
           }
         }
         __syncwarp();   // the staging rows are overwritten by the next block
@@ -417,6 +522,42 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
+}
+
+// planes[p][line][at] = term p of x[line][at], lines `ld_out` elements apart and planes `plane`; one flag per
+// block for an infinity or a value from 2^127 on.  Bound by memory: 4 bytes in, 6 out per element.
+__global__ void __launch_bounds__(256) f3_split_kernel(const float *__restrict__ x, int64_t lines, int cols, int64_t ld, int vec,
+                                                       __nv_bfloat16 *planes, int ld_out, int64_t plane, uint32_t *big) {
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  const int quads = (cols + 3) / 4;
+  const int64_t total = lines * quads, stride = (int64_t)gridDim.x * blockDim.x;
+  float top = 0.f;
+#pragma unroll 4
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
+    const int64_t line = e / quads;
+    const int at = (int)(e - line * quads) * 4;
+    const float *src = x + line * ld + at;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (vec && at + 4 <= cols) {
+      v = *reinterpret_cast<const float4 *>(src);
+    } else {
+      v.x = src[0];
+      if (at + 1 < cols) v.y = src[1];
+      if (at + 2 < cols) v.z = src[2];
+      if (at + 3 < cols) v.w = src[3];
+    }
+    uint2 h, m, l;
+    split3(v.x, v.y, h.x, m.x, l.x);
+    split3(v.z, v.w, h.y, m.y, l.y);
+    __nv_bfloat16 *dst = planes + line * ld_out + at;   // ld_out is a multiple of 8: room for a whole quad
+    *reinterpret_cast<uint2 *>(dst) = h;
+    *reinterpret_cast<uint2 *>(dst + plane) = m;
+    *reinterpret_cast<uint2 *>(dst + 2 * plane) = l;
+    top = fmax3(top, fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+  }
+  const int any = __syncthreads_or(top >= 1.7014118346046923e38f);
+  if (threadIdx.x == 0) big[blockIdx.x] = any;
 }
 
 // C = finish(sum of the slabs in split order)
@@ -458,35 +599,45 @@ __global__ void __launch_bounds__(256) gemm_f32_reduce_kernel(const GemmF32TcArg
   }
 }
 
-template <bool A_MN, bool B_MN, int BN>
-static int f3_launch(const GemmF32TcArgs &g, int grid) {
+template <bool A_MN, bool B_MN, int BN, bool SPLIT_B>
+static int f3_launch(const CUtensorMap &tb, const GemmF32TcArgs &g, int grid) {
   static int attr = -1;
   if (attr != g_init_epoch) {
-    ALPHA_CUDA(cudaFuncSetAttribute(gemm_f32_tc_kernel<A_MN, B_MN, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    ALPHA_CUDA(cudaFuncSetAttribute(gemm_f32_tc_kernel<A_MN, B_MN, BN, SPLIT_B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     F3Layout<BN>::DYN));
     attr = g_init_epoch;
   }
-  ALPHA_CUDA(launch_overlapped(OVL_GEMM, gemm_f32_tc_kernel<A_MN, B_MN, BN>, dim3(grid), dim3(F3_THREADS),
-                               F3Layout<BN>::DYN, g));
+  ALPHA_CUDA(launch_overlapped(OVL_GEMM, gemm_f32_tc_kernel<A_MN, B_MN, BN, SPLIT_B>, dim3(grid), dim3(F3_THREADS),
+                               F3Layout<BN>::DYN, tb, g));
   ALPHA_LAUNCHED();
   return 0;
 }
 
-// Tile width and number of K splits: the pair that minimises waves x (K steps + fixed part) plus the
-// pass that adds the splits, in cycles of one SM.
-static void f3_plan(int64_t M, int64_t N, int64_t kblocks, int64_t batch, int &bn, int &splits) {
+// Tile width, number of K splits, and whether B is split by a kernel of its own: the choice of least modelled
+// time, in microseconds, fitted to a sweep of M = 1 ... 16384 over the products of models of width 64 to 384
+// (fixed part and K step of a launch, epilogues that read or transform, the second launch and traffic of a
+// split sum, the extra launch and traffic of a split B).  E.g. 16384 x 4096 x 384: 335 us with B split in the
+// kernel, 292 outside; 256 x 768 x 256: 9.0 and 10.8; 768 x 256 x 16384 in 12 splits: 46 and 51.
+static void f3_plan(int64_t M, int64_t N, int64_t K, int64_t batch, bool epilogue, int &bn, int &splits, bool &split_b) {
+  const int64_t kblocks = (K + F3_BK - 1) / F3_BK;
   double best = 1e300;
   for (int w = 128; w >= 64; w -= 64) {
     const int64_t tiles = ((M + F3_BM - 1) / F3_BM) * ((N + w - 1) / w) * batch;
-    const double per_kb = w == 128 ? 2300.0 : 1500.0, fixed = 4000.0;
-    for (int64_t sp = 1; sp <= kblocks && sp <= 64; sp++) {
-      const int64_t waves = (tiles * sp + g_sm_count - 1) / g_sm_count, kb = (kblocks + sp - 1) / sp;
-      double t = (double)waves * (double)kb * per_kb + fixed;
-      if (sp > 1) t += 4000.0 + (double)(2 * sp + 1) * (double)M * (double)N * (double)batch * 4.0 / 2700.0;
-      if (t < best) {
-        best = t;
-        bn = w;
-        splits = (int)sp;
+    for (int sb = 0; sb <= (batch == 1 ? 1 : 0); sb++) {
+      const double step = w == 128 ? (sb ? 1.74 : 2.0) : (sb ? 1.2 : 1.45), fixed = w == 128 ? 4.7 : 3.8;
+      const double once = fixed + (sb ? 2.0 + 10.0 * (double)N * (double)K / 4.0e6 : 0.0);
+      const double tail = !epilogue ? 0.0 : w == 128 ? 5.5 : 2.5;   // of a tile's epilogue, beyond a plain store
+      for (int64_t sp = 1; sp <= kblocks && sp <= 64 && (sp == 1 || tiles * sp <= 4 * g_sm_count); sp++) {
+        const int64_t waves = (tiles * sp + g_sm_count - 1) / g_sm_count, kb = (kblocks + sp - 1) / sp;
+        double t = once + (double)(waves * kb) * step;
+        if (sp == 1) t += (double)waves * tail;
+        else t += 2.9 + 0.06 * (double)sp + (double)(sp + 1) * (double)M * (double)N * (double)batch * 4.0 / 5.0e6;
+        if (t < best) {
+          best = t;
+          bn = w;
+          splits = (int)sp;
+          split_b = sb != 0;
+        }
       }
     }
   }
@@ -505,7 +656,8 @@ int gemm_f32_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_
   g.M = (int)M; g.N = (int)N; g.K = (int)K; g.batch = (int)batch;
   g.kblocks = (int)((K + F3_BK - 1) / F3_BK);
   int bn = 128, splits = 1;
-  f3_plan(M, N, g.kblocks, batch, bn, splits);
+  bool split_b = false;
+  f3_plan(M, N, K, batch, epilogue != ALPHA_EPI_NONE || accumulate, bn, splits, split_b);
   g.kb_per_split = (g.kblocks + splits - 1) / splits;
   g.splits = splits = (g.kblocks + g.kb_per_split - 1) / g.kb_per_split;   // drop empty splits
   g.tiles_m = (int)((M + F3_BM - 1) / F3_BM);
@@ -530,11 +682,39 @@ int gemm_f32_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_
   }
   const int64_t units = (int64_t)g.tiles_m * g.tiles_n * splits * batch;
   const int grid = (int)(units < g_sm_count ? units : g_sm_count);
+  // B's planes in a pass of their own when enough tiles share them
+  CUtensorMap tb;
+  memset(&tb, 0, sizeof(tb));
+  void *bws = nullptr;
+  if (split_b) {
+    const int64_t lines = b_mn ? K : N, cols = b_mn ? N : K, ld_out = (cols + 7) / 8 * 8, plane = lines * ld_out;
+    const int blocks = grid_for(lines * ((cols + 3) / 4), 256, 4);
+    if (pool_alloc((size_t)plane * 6 + (size_t)blocks * 4, &bws) ||
+        encode_tmap_3d_bf16(&tb, bws, cols, lines, 3, ld_out, plane, 64, b_mn ? 64 : bn, 1)) {
+      if (bws) pool_free(bws);
+      if (ws) pool_free(ws);
+      return 1;
+    }
+    uint32_t *flags = reinterpret_cast<uint32_t *>((char *)bws + plane * 6);
+    g.b_big = flags;
+    g.n_b_big = blocks;
+    const cudaError_t e = launch_overlapped(OVL_GEMM, f3_split_kernel, dim3(blocks), dim3(256), 0, g.B, lines, (int)cols, ldb, g.vec_b,
+                                            (__nv_bfloat16 *)bws, (int)ld_out, plane, flags);
+    if (e != cudaSuccess) {
+      pool_free(bws);
+      if (ws) pool_free(ws);
+      return set_error("alpha_gemm: split launch -> %s", cudaGetErrorString(e));
+    }
+    g_launches++;
+  }
   int rc;
-  if (bn == 128)
-    rc = a_mn ? f3_launch<true, true, 128>(g, grid) : b_mn ? f3_launch<false, true, 128>(g, grid) : f3_launch<false, false, 128>(g, grid);
-  else
-    rc = a_mn ? f3_launch<true, true, 64>(g, grid) : b_mn ? f3_launch<false, true, 64>(g, grid) : f3_launch<false, false, 64>(g, grid);
+#define F3_LAYOUT(BNV, SB)                                                                                         \
+  (a_mn ? f3_launch<true, true, BNV, SB>(tb, g, grid)                                                              \
+        : b_mn ? f3_launch<false, true, BNV, SB>(tb, g, grid) : f3_launch<false, false, BNV, SB>(tb, g, grid))
+  if (bn == 128) rc = split_b ? F3_LAYOUT(128, true) : F3_LAYOUT(128, false);
+  else rc = split_b ? F3_LAYOUT(64, true) : F3_LAYOUT(64, false);
+#undef F3_LAYOUT
+  if (bws) pool_free(bws);
   if (rc == 0 && splits > 1) {
     const int v = out_vec && N % 4 == 0;
     const cudaError_t e = launch_overlapped(OVL_SPLITK, gemm_f32_reduce_kernel,

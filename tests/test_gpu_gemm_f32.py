@@ -54,7 +54,9 @@ def operands(layout, M, N, K, seed, scale=1.0):
 @pytest.mark.parametrize("layout", [0, 1, 2])
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 64, 64), (3, 5, 7), (127, 65, 63), (128, 128, 64), (129, 129, 65),
                                    (256, 192, 64), (48, 1152, 384), (200, 96, 1536), (257, 512, 130),
-                                   (1024, 1024, 256), (96, 64, 16384), (4096, 72, 100), (2500, 1300, 40)])
+                                   (1024, 1024, 256), (96, 64, 16384), (4096, 72, 100), (2500, 1300, 40),
+                                   # large enough that B is split by a kernel of its own: rows of 16 bytes and not
+                                   (5000, 1032, 392), (4100, 1030, 390), (3000, 1500, 700)])
 def test_against_64_bits(B, layout, M, N, K):
     a, b, (sa, sb) = operands(layout, M, N, K, M + N + K)
     got = product(B, layout, sa, sb, M, N, K)
@@ -93,25 +95,27 @@ def test_epilogues(B, M, N, K, epilogue, accumulate):
 
 
 @pytest.mark.parametrize("layout", [0, 1, 2])
-@pytest.mark.parametrize("K", [100, 2048])
-def test_infinities_and_huge_values(B, layout, K):
+@pytest.mark.parametrize("M,N,K", [(140, 70, 100), (140, 70, 2048), (4100, 1030, 390)])   # one split, many, B on its own
+def test_infinities_and_huge_values(B, layout, M, N, K):
     """inf * finite, inf * 0, values that round to inf in 16 bits and NaN: as an fmaf chain gives them."""
-    M, N = 140, 70
     a, b, _ = operands(1, M, N, K, 3)
     a[5, 9], a[6, 10], a[131, 3], a[7, 1] = np.inf, -np.inf, 3.4e38, np.nan
     b[:, 2] = np.where(np.arange(K) % 2, 0.0, b[:, 2])
     b[9, 4], b[3, :] = 0.0, 0.25
+    b[50, 33] = -np.inf                        # in the other operand too
     a, b = (x.astype(np.float32).astype(np.float64) for x in (a, b))
     stored = {0: (a, b.T), 1: (a, b), 2: (a.T, b)}[layout]
     got = product(B, layout, *stored, M, N, K)
     with np.errstate(invalid="ignore"):
         want = a @ b
+        off = np.abs(got - want)
     assert np.array_equal(np.isnan(got), np.isnan(want))
     assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
     fin = np.isfinite(want)
     finite = lambda x: np.where(np.isfinite(x), x, 0.0)
     # the recomputed elements are a chain of K
-    assert np.all(np.abs(got - want)[fin] <= (bound(finite(a), b, K) + K * U * (np.abs(finite(a)) @ np.abs(b)))[fin])
+    a, b = finite(a), finite(b)
+    assert np.all(off[fin] <= (bound(a, b, K) + K * U * (np.abs(a) @ np.abs(b)))[fin])
 
 
 @pytest.mark.parametrize("exponent", [-100, -30, 30, 100])
