@@ -270,6 +270,33 @@ __device__ __forceinline__ void fix_scores(float (&acc)[NN][4], const T *a, cons
     }
 }
 
+// tanh: by its Taylor series up to y^13 where the whole warp's arguments lie within 0.35 (truncation below 2e-9
+// of the value; soft-capped scores of a trained or fresh model rarely leave it), else tanhf, whose two branches
+// a warp with mixed arguments runs both of.  Default model in bf16 4.69 -> 4.59 ms a step, in fp32 8.39 -> 8.33.
+constexpr float TANH_SERIES_LIMIT = 0.35f;
+template <bool SERIES>
+__device__ __forceinline__ float cap_tanh(float y) {
+  if (!SERIES) return tanhf(y);
+  const float u = y * y;
+  float t = fmaf(u, 21844.f / 6081075.f, -1382.f / 155925.f);
+  t = fmaf(u, t, 62.f / 2835.f);
+  t = fmaf(u, t, -17.f / 315.f);
+  t = fmaf(u, t, 2.f / 15.f);
+  t = fmaf(u, t, -1.f / 3.f);
+  return fmaf(y * u, t, y);
+}
+// Whether every raw score of the warp's tile takes the series (a NaN stays one either way).
+template <int NN>
+__device__ __forceinline__ bool series_fits(const float (&s)[NN][4], float cap_arg) {
+  float top = 0.f;
+#pragma unroll
+  for (int n = 0; n < NN; n++) {
+    top = tc::fmax3(top, fabsf(s[n][0]), fabsf(s[n][1]));
+    top = tc::fmax3(top, fabsf(s[n][2]), fabsf(s[n][3]));
+  }
+  return __all_sync(0xffffffffu, top * fabsf(cap_arg) <= TANH_SERIES_LIMIT);
+}
+
 // Four lanes of a quad share a row.
 __device__ __forceinline__ float quad_max(float v) {
   v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
@@ -321,16 +348,32 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_fwd_kernel(const AttnArgs a
     float s[8][4];
     score_product<T, D, 8>(s, q_u, warp * 16, k_u, 0, 0, groups, lane);
     if (L::NT > 1 && big) fix_scores<T, D, 8>(s, qp, kp, a.q_st, a.q_st, q0 + warp * 16, k0, a.T);
+    if (a.cap > 0.f) {
+      if (series_fits(s, a.cap_arg)) {
+#pragma unroll
+        for (int n = 0; n < 8; n++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) s[n][i] = a.cap * cap_tanh<true>(s[n][i] * a.cap_arg);
+      } else {
+#pragma unroll
+        for (int n = 0; n < 8; n++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) s[n][i] = a.cap * cap_tanh<false>(s[n][i] * a.cap_arg);
+      }
+    } else {
+#pragma unroll
+      for (int n = 0; n < 8; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[n][i] *= a.scale;
+    }
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int n = 0; n < 8; n++)
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const int qi = row0 + (i >> 1) * 8, kj = k0 + n * 8 + (lane & 3) * 2 + (i & 1);
-        float x = a.cap > 0.f ? a.cap * tanhf(s[n][i] * a.cap_arg) : s[n][i] * a.scale;
-        if (kj > qi || kj >= a.T) x = -INFINITY;
-        s[n][i] = x;
-        mx[i >> 1] = fmaxf(mx[i >> 1], x);
+        if (kj > qi || kj >= a.T) s[n][i] = -INFINITY;
+        mx[i >> 1] = fmaxf(mx[i >> 1], s[n][i]);
       }
     float corr[2];
 #pragma unroll
@@ -384,11 +427,12 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(AttnArgs a, int D, int6
 }
 
 // From raw score s and dP of (query qi, key kj): P and dS.
+template <bool SERIES>
 __device__ __forceinline__ void p_and_ds(const AttnArgs &a, float s, float dp, float lse, float delta, int qi, int kj,
                                          float &p, float &ds) {
   float x = s * a.scale, dcap = 1.f;
   if (a.cap > 0.f) {
-    const float th = tanhf(s * a.cap_arg);
+    const float th = cap_tanh<SERIES>(s * a.cap_arg);
     x = a.cap * th;
     dcap = 1.f - th * th;
   }
@@ -442,13 +486,23 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_bwd_dkv_kernel(const AttnAr
         fix_scores<T, D, 4>(s, kp, qp, a.q_st, a.q_st, k0 + warp * 16, q0 + c, a.T);
         fix_scores<T, D, 4>(dp, vp, dop, a.q_st, a.o_st, k0 + warp * 16, q0 + c, a.T);
       }
+      if (series_fits(s, a.cap_arg)) {   // also without a cap: cap_arg is 0 then
 #pragma unroll
-      for (int n = 0; n < 4; n++)
+        for (int n = 0; n < 4; n++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const int qc = c + n * 8 + (lane & 3) * 2 + (i & 1);
-          p_and_ds(a, s[n][i], dp[n][i], lse_s[qc], delta_s[qc], q0 + qc, row0 + (i >> 1) * 8, s[n][i], dp[n][i]);
-        }
+          for (int i = 0; i < 4; i++) {
+            const int qc = c + n * 8 + (lane & 3) * 2 + (i & 1);
+            p_and_ds<true>(a, s[n][i], dp[n][i], lse_s[qc], delta_s[qc], q0 + qc, row0 + (i >> 1) * 8, s[n][i], dp[n][i]);
+          }
+      } else {
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const int qc = c + n * 8 + (lane & 3) * 2 + (i & 1);
+            p_and_ds<false>(a, s[n][i], dp[n][i], lse_s[qc], delta_s[qc], q0 + qc, row0 + (i >> 1) * 8, s[n][i], dp[n][i]);
+          }
+      }
       LeftTerms<2> w;
       w.set(s);
       output_product<T, D, 2, false>(dv, w, do_u, c, from, 2, 1.f, 1.f, lane);   // dV[key] += sum_q P[q][key] dO[q]
@@ -515,14 +569,22 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_bwd_dq_kernel(const AttnArg
         fix_scores<T, D, 4>(s, qp, kp, a.q_st, a.q_st, q0 + warp * 16, k0 + c, a.T);
         fix_scores<T, D, 4>(dp, dop, vp, a.o_st, a.q_st, q0 + warp * 16, k0 + c, a.T);
       }
+      float p;
+      if (series_fits(s, a.cap_arg)) {   // also without a cap: cap_arg is 0 then
 #pragma unroll
-      for (int n = 0; n < 4; n++)
+        for (int n = 0; n < 4; n++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          float p;
-          p_and_ds(a, s[n][i], dp[n][i], lse[i >> 1], delta[i >> 1], row0 + (i >> 1) * 8,
-                   k0 + c + n * 8 + (lane & 3) * 2 + (i & 1), p, dp[n][i]);
-        }
+          for (int i = 0; i < 4; i++)
+            p_and_ds<true>(a, s[n][i], dp[n][i], lse[i >> 1], delta[i >> 1], row0 + (i >> 1) * 8,
+                           k0 + c + n * 8 + (lane & 3) * 2 + (i & 1), p, dp[n][i]);
+      } else {
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            p_and_ds<false>(a, s[n][i], dp[n][i], lse[i >> 1], delta[i >> 1], row0 + (i >> 1) * 8,
+                            k0 + c + n * 8 + (lane & 3) * 2 + (i & 1), p, dp[n][i]);
+      }
       LeftTerms<2> w;
       w.set(dp);
       output_product<T, D, 2, false>(dq, w, k_u, c, 0, to, 1.f, 1.f, lane);   // dQ[q] += sum_key dS[q][key] K[key]

@@ -115,4 +115,9 @@ def test_infinite_scores_meet_the_cap(B):
     q[0, 70, 4] = np.inf
     got = np.array(B.flashAttention(*(B.upload(t, "f32") for t in (q, k, v)), T, 0.2, 30.0)["output"].data)
     assert np.allclose(got[0, 70], v[0, :71].mean(0), rtol=1e-5, atol=1e-6)     # every score at the cap: the mean
-    assert np.array_equal(np.delete(got, 70, 1), np.delete(clean, 70, 1))
+    # rows in the same warp go through tanhf with it instead of the series: 2 ulp of a score below 8 each, so P and the
+    # outputs move by at most 4 * 8 * 2^-23 of |v|; all other rows are the same bits
+    warp = list(range(64, 80))
+    assert np.array_equal(np.delete(got, warp, 1), np.delete(clean, warp, 1))
+    near = np.delete(np.array(warp), 6)
+    assert np.all(np.abs(got[:, near] - clean[:, near]) <= 32 * 2.0 ** -23 * np.abs(v).max())
