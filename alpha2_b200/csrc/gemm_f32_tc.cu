@@ -673,9 +673,13 @@ int gemm_f32_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_
   g.vec_c = out_vec;
   g.err = tc_error_word();
   void *ws = nullptr;
+  if (splits > 1 && pool_alloc((size_t)splits * batch * M * N * sizeof(float), &ws)) {
+    ws = nullptr;   // no room for the slabs: one split needs none
+    g.splits = splits = 1;
+    g.kb_per_split = g.kblocks;
+  }
   if (splits > 1) {
     g.split_c = batch * M * N;
-    if (pool_alloc((size_t)splits * g.split_c * sizeof(float), &ws)) return 1;
     g.C = (float *)ws; g.ldc = N; g.batch_c = M * N;
     g.epilogue = ALPHA_EPI_NONE; g.accumulate = 0;
     g.vec_c = N % 4 == 0;
@@ -689,12 +693,18 @@ int gemm_f32_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_
   if (split_b) {
     const int64_t lines = b_mn ? K : N, cols = b_mn ? N : K, ld_out = (cols + 7) / 8 * 8, plane = lines * ld_out;
     const int blocks = grid_for(lines * ((cols + 3) / 4), 256, 4);
-    if (pool_alloc((size_t)plane * 6 + (size_t)blocks * 4, &bws) ||
-        encode_tmap_3d_bf16(&tb, bws, cols, lines, 3, ld_out, plane, 64, b_mn ? 64 : bn, 1)) {
-      if (bws) pool_free(bws);
+    if (pool_alloc((size_t)plane * 6 + (size_t)blocks * 4, &bws)) {
+      bws = nullptr;   // no room for the planes: the operand warps split B themselves
+      split_b = false;
+    } else if (encode_tmap_3d_bf16(&tb, bws, cols, lines, 3, ld_out, plane, 64, b_mn ? 64 : bn, 1)) {
+      pool_free(bws);
       if (ws) pool_free(ws);
       return 1;
     }
+  }
+  if (split_b) {
+    const int64_t lines = b_mn ? K : N, cols = b_mn ? N : K, ld_out = (cols + 7) / 8 * 8, plane = lines * ld_out;
+    const int blocks = grid_for(lines * ((cols + 3) / 4), 256, 4);
     uint32_t *flags = reinterpret_cast<uint32_t *>((char *)bws + plane * 6);
     g.b_big = flags;
     g.n_b_big = blocks;

@@ -885,6 +885,15 @@ int gemm_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M,
   int splits = plan.splits;
   g.kb_per_split = (g.kblocks + splits - 1) / splits;
   splits = (g.kblocks + g.kb_per_split - 1) / g.kb_per_split;  // drop empty splits
+  g.m_pad = g.tiles_m * tile_m;
+  void *ws = nullptr;
+  // one slab per split, padded to whole tiles so that a tile's rows below the matrix land in
+  // the slab's own padding (TMA clips at the tensor's edge, not at a slab's)
+  if (splits > 1 && pool_alloc((size_t)splits * g.m_pad * N * sizeof(float), &ws)) {
+    ws = nullptr;   // no room for the slabs: one split needs none
+    splits = 1;
+    g.kb_per_split = g.kblocks;
+  }
   g.splits = splits;
   // C += A*B with nothing else in the epilogue is the residual-add epilogue with C as its own
   // addend: the old tile arrives by TMA in the staging buffer the new one leaves from, instead
@@ -896,12 +905,7 @@ int gemm_tc_launch(int layout, alpha_buf A, alpha_buf B, alpha_buf C, int64_t M,
     ld_aux = ldc;
     accumulate = 0;
   }
-  void *ws = nullptr;
-  g.m_pad = g.tiles_m * tile_m;
   if (splits > 1) {
-    // one slab per split, padded to whole tiles so that a tile's rows below the matrix land in
-    // the slab's own padding (TMA clips at the tensor's edge, not at a slab's)
-    if (pool_alloc((size_t)splits * g.m_pad * N * sizeof(float), &ws)) return 1;
     g.C = ws; g.ldc = N; g.out_f32 = 1; g.epilogue = ALPHA_EPI_NONE; g.accumulate = 0;
   } else {
     g.C = ptr<void>(C); g.ldc = ldc; g.out_f32 = out_dtype == ALPHA_F32;

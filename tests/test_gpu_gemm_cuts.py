@@ -25,7 +25,8 @@ def rounded(x):
 
 @pytest.mark.parametrize("layout", [0, 1, 2])
 @pytest.mark.parametrize("M,N,K", [(1, 136, 768), (8, 256, 4096), (129, 257, 64), (200, 768, 3072), (130, 1160, 136),
-                                   (777, 136, 1536), (1030, 520, 200), (2336, 776, 768)])
+                                   (777, 136, 1536), (1030, 520, 200), (2336, 776, 768),
+                                   (72, 131, 2048)])      # split, rows of the slabs not 16 bytes
 @pytest.mark.parametrize("epilogue,accumulate,out", [(0, 0, "bf16"), (0, 1, "f32"), (1, 0, "bf16"), (2, 0, "bf16"),
                                                      (3, 0, "bf16")])
 def test_against_64_bits(B, layout, M, N, K, epilogue, accumulate, out):
