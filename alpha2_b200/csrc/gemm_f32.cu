@@ -2,10 +2,10 @@
 // reference accumulates each dot product in a double and rounds once,
 // packages/tensor/src/cpu_ref.ts:246-254).  The products run on the tensor cores as sums of
 // exact bf16 term products (gemm_f32_tc.cu); the kernel here, on the FMA pipes, takes what that
-// one does not: an empty sum (K = 0, epilogues included) and outputs of more than 2^25 tiles.  Arbitrary element strides cover the
-// three layouts of the Backend interface — A*B, A*B^T (matmulTransposed) and A^T*B
-// (matmulTransposedA), packages/core/src/interfaces.ts:53,111-112 — and batched matmul
-// with broadcastable batch strides for the unfused attention branch
+// one does not: an empty sum (K = 0, epilogues included) and outputs of more than 2^25 tiles.
+// Arbitrary element strides cover the three layouts of the Backend interface — A*B, A*B^T
+// (matmulTransposed) and A^T*B (matmulTransposedA), packages/core/src/interfaces.ts:53,111-112 —
+// and batched matmul with broadcastable batch strides for the unfused attention branch
 // (packages/model/src/gpt.ts:256-279).
 //
 // 64x64x16 shared-memory tiles, 256 threads, 4x4 outputs per thread.
