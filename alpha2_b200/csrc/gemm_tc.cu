@@ -816,7 +816,7 @@ static int splitk_reduce_launch(SplitkReduceArgs r, int out_dtype) {
 // products of models of width 256 to 768): a launch costs `fixed` and `step` per wave and K step of 64,
 // and splits cost a second launch and the slabs' traffic.  A single CTA with a 128 x 128 tile starts and
 // ends soonest, so it takes what fits in a wave or two; a pair moves the fewest operand bytes per flop and
-// takes the rest, and what the model finds within a tenth (inside a step launches overlap, which hides
+// takes the rest, and unsplit what the model finds within a tenth (inside a step launches overlap, which hides
 // part of `fixed`: a step of width 384 at 8192 tokens lost 0.8 % without that margin).  E.g. 200 x 768 x 3072 with the residual: 13.0 us by pairs, 10.6 as 128 x 128 in six splits;
 // 2331 x 768 x 768: 12.9 and 9.4; 16384 x 2304 x 768: 40.2 and 65.7.
 struct TcPlan {
@@ -836,7 +836,7 @@ static TcPlan tc_plan(int64_t M, int64_t N, int64_t kblocks, bool can_split) {
       const int64_t waves = (tiles * sp + slots - 1) / slots, kb = (kblocks + sp - 1) / sp;
       double t = c.fixed + (double)(waves * kb) * c.step;
       if (sp > 1) t += 2.6 + (double)(sp + 1) * (double)M * (double)N * 4.0 / 5.0e6;
-      if (c.pair) t *= 0.9;
+      if (c.pair && sp == 1) t *= 0.9;
       if (t < best_t) {
         best_t = t;
         best = TcPlan{c.pair, c.bn, (int)sp};
